@@ -27,7 +27,8 @@ LIB = os.path.join(HERE, "lib")
 OBJ = os.path.join(ROOT, "_build", "obj")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVFLAGS = ARCH + ["-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
+# --split-compile: a source's many transform kernels are optimised on several threads
+NVFLAGS = ARCH + ["--split-compile=8", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
                   "--expt-relaxed-constexpr", "-I" + CSRC, "-I" + os.path.join(ROOT, "include")]
 LIBNAME = os.path.join(LIB, "libtroy_b200.so")
 

@@ -37,6 +37,7 @@ Context::~Context() {
     if (d_drop) cudaFree(d_drop);
     if (d_mods) cudaFree(d_mods);
     if (d_tables) cudaFree(d_tables);
+    if (d_fp_tables) cudaFree(d_fp_tables);
     cudaSetDevice(prev);
 }
 
@@ -71,6 +72,53 @@ static bool build_ntt_tables(uint64_t q, int logn, std::vector<ulonglong2> &fwd,
     m.sroot = mulmod(last, m.inv_n, q);
     m.sroot_quo = shoup(m.sroot, q);
     return true;
+}
+
+// FP64 twiddles of one modulus from its integer tables (fp64mod.cuh): N forward words, N
+// inverse words, N / 16 forward and N / 16 inverse pairs.
+__global__ void fp_tables_kernel(const ulonglong2 *__restrict__ roots, const ulonglong2 *__restrict__ inv_roots,
+                                 uint64_t q, double qinv, int logn, double *__restrict__ w) {
+    const uint32_t n = 1u << logn, np = n >> 4;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint32_t f = i ? fp_fwd_index(i, logn) : 0, v = i ? fp_inv_index(i, logn) : 0;
+    const double a = fp_centred(roots[i].x, q), b = fp_centred(inv_roots[i].x, q);
+    double2 *p = reinterpret_cast<double2 *>(w + 2 * n);
+    w[f] = a;
+    w[n + v] = b;
+    if (f < np) p[f] = make_double2(a, __dmul_rn(a, qinv));
+    if (v >= n - np) p[np + v - (n - np)] = make_double2(b, __dmul_rn(b, qinv));
+}
+
+// The FP64 tables of every table modulus below 2^50, for the degrees whose transforms
+// have an FP64 form: the twiddles of each, then the FpMod descriptors.
+static cudaError_t build_fp_tables(Context &c) {
+    if (c.logn < FP_MIN_LOGN || c.logn > FP_MAX_LOGN) return cudaSuccess;
+    std::vector<FpMod> desc;
+    std::vector<size_t> at;
+    for (size_t i = 0; i < c.h_mods.size(); i++)
+        if (c.h_mods[i].value < FP_MAX_Q) at.push_back(i);
+    if (at.empty()) return cudaSuccess;
+    const size_t n = c.n, words = 2 * n + n / 4;   // and 2 (N / 16) pairs
+    cudaError_t e = cudaMalloc(&c.d_fp_tables, at.size() * (words * sizeof(double) + sizeof(FpMod)));
+    if (e != cudaSuccess) return e;
+    FpMod *d_desc = reinterpret_cast<FpMod *>(c.d_fp_tables + at.size() * words);
+    auto centred = [](uint64_t w, uint64_t q) { return w > q / 2 ? -(double)(q - w) : (double)w; };
+    for (size_t k = 0; k < at.size() && e == cudaSuccess; k++) {
+        Mod &m = c.h_mods[at[k]];
+        double *w = c.d_fp_tables + words * k;
+        const double2 *p = reinterpret_cast<const double2 *>(w + 2 * n);
+        const double qinv = 1.0 / (double)m.value;
+        fp_tables_kernel<<<(unsigned)(n / 256), 256>>>(m.roots, m.inv_roots, m.value, qinv, c.logn, w);
+        e = cudaGetLastError();
+        desc.push_back(FpMod{w, w + n, p, p + n / 16, (double)m.value, qinv, centred(m.inv_n, m.value),
+                             centred(m.sroot, m.value)});
+        m.fp = d_desc + k;
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(d_desc, desc.data(), desc.size() * sizeof(FpMod), cudaMemcpyHostToDevice);
+    // the legacy stream's kernels finish before the context is used on any stream
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    return e;
 }
 
 int build_rns_levels(Context &c);  // rns.cu
@@ -134,7 +182,8 @@ int context_create(int scheme, uint64_t n, const uint64_t *moduli, int count, ui
         c->h_mods[i].roots = c->d_tables + (2 * i) * n;
         c->h_mods[i].inv_roots = c->d_tables + (2 * i + 1) * n;
     }
-    e = cudaMalloc(&c->d_mods, nm * sizeof(Mod));
+    e = build_fp_tables(*c);
+    if (e == cudaSuccess) e = cudaMalloc(&c->d_mods, nm * sizeof(Mod));
     if (e == cudaSuccess) e = cudaMemcpy(c->d_mods, c->h_mods.data(), nm * sizeof(Mod), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         delete c;
@@ -174,7 +223,9 @@ struct PlainNttOp {
         const int l = limb_block % limbs;
         Ctx c;
         c.lm = make_limb(mods[first + l], sb);
-        c.slack = (FWD && !lazy && c.lm.q < (1ull << 60)) ? SLACK_M : 0;
+        // full outputs of whole limbs: the FP64 form where the modulus has one
+        if (!lazy && !log_nsub) c.lm.fp = fp_form(mods[first + l], !FWD);
+        c.slack = (FWD && !lazy && !c.lm.fp && c.lm.q < (1ull << 60)) ? SLACK_M : 0;
         c.islack = !FWD && !lazy;
         const size_t off = ((size_t)limb_block << (logb + log_nsub)) + ((size_t)sb << logb);
         c.in = in + off;
@@ -271,9 +322,11 @@ static int ntt_plain(const Context &c, const uint64_t *in, uint64_t *out, uint64
     const uint64_t total = polys * (uint64_t)limbs;
     const int logn = c.logn;
     // limbs up to 2^14 in one launch, and 2^15 inverse transforms on two-CTA clusters;
-    // longer limbs (and 2^15 forward transforms, measured faster so) split into global
-    // top stages and 2^14 sub-blocks
-    const int logb = (logn <= MAX_LOGB || (!FWD && logn == PAIR_LOGN)) ? logn : MAX_LOGB;
+    // longer limbs (and 2^15 forward transforms in integer form, measured faster so) split
+    // into global top stages and 2^14 sub-blocks
+    bool fp = !lazy && logn == PAIR_LOGN;
+    for (int l = 0; l < limbs && fp; l++) fp = c.h_mods[first + l].fp != nullptr;
+    const int logb = (logn <= MAX_LOGB || ((!FWD || fp) && logn == PAIR_LOGN)) ? logn : MAX_LOGB;
     const int h = logn - logb;
     if ((total << h) > 0x7fffffffULL || (h > 0 && total > 65535))
         return set_error(TB_ERR_INVALID_ARGUMENT, "too many limbs in one launch");

@@ -99,6 +99,7 @@ struct Context {
     std::vector<Mod> h_mods;          // host copy (device table pointers inside)
     Mod *d_mods = nullptr;
     ulonglong2 *d_tables = nullptr;
+    double *d_fp_tables = nullptr;    // FP64 twiddles of the moduli below 2^50 (fp64mod.cuh)
     std::vector<RnsLevel> levels;     // levels[L] for L = 1 .. chain.size()
     DropC *d_drop = nullptr;          // [(Lfull) * K + j], K = chain.size()
     Mod t_mod{};                      // plain modulus (Barrett ratio only), value 0 for CKKS

@@ -103,6 +103,7 @@ struct StridedNttOp {
         const int p = b / limbs, l = b % limbs;
         Ctx c;
         c.lm = make_limb(mods[first + l], 0);
+        if (!FWD && !lazy) c.lm.fp = fp_form(mods[first + l]);
         c.islack = !FWD && !lazy;
         c.in = in + (size_t)p * istride + ((size_t)l << logn);
         c.out = out + (size_t)p * ostride + ((size_t)l << logn);
@@ -136,6 +137,7 @@ struct ModUpOp {
     const Mod *mods;
     const uint64_t *chain;    // device copy of chain values (for the reduce test)
     int L, K, ckks, logn;
+    int B;                    // ciphertexts of the launch
     // Up to 15 digits are summed unreduced by the 128-bit inner products: below 4q (a
     // 61-bit q), below 16 q (q < 2^60, deferred reductions), or, for q < 2^57 in the
     // one-CTA transform (no subtraction, estimated quotients), below 2^61 + 56 q <
@@ -154,16 +156,25 @@ struct ModUpOp {
         int slack;
     };
     __device__ Ctx ctx(int b) const {
-        const int P = ckks ? L * L : L * (L + 1);
-        const int cb = b / P, p = b % P;
-        int j, i;
-        if (ckks) {
-            j = p / L;
-            const int ii = p % L;
-            i = ii + (ii >= j);
+        // the special prime's limbs first (integer form, the longest): the cheaper limbs
+        // fill the last wave; the others digit by digit, so that a digit's CTAs find it in L2
+        int cb, j, i;
+        const int special = L * B, per = ckks ? L * (L - 1) : L * L;
+        if (b < special) {
+            i = L;
+            cb = b / L;
+            j = b % L;
         } else {
-            j = p / (L + 1);
-            i = p % (L + 1);
+            const int r = b - special, p = r % per;
+            cb = r / per;
+            if (ckks) {   // digit i of modulus i is the target itself
+                j = p / (L - 1);
+                i = p % (L - 1);
+                i += i >= j;
+            } else {
+                j = p / L;
+                i = p % L;
+            }
         }
         const int mi = i == L ? K - 1 : i;
         const Mod &m = mods[mi];
@@ -172,9 +183,11 @@ struct ModUpOp {
         c.ratio_hi = m.ratio_hi;
         // the transform's input: any digit word in the no-subtraction form, below 4q in
         // the others (a Barrett remainder in [0, 2q) when q_j is larger)
+        // the FP64 form (canonical outputs) takes words below 2^49, or the remainder
+        c.lm.fp = fp_form(m);
         const bool wide = L <= LAZY_MAX_L && logn <= MAX_LOGB && m.value < (1ull << 57);
         c.slack = wide ? SLACK_WIDE : m.value < (1ull << 60) ? SLACK_M : 0;
-        c.reduce = !wide && mods[j].value > 4 * m.value;
+        c.reduce = c.lm.fp ? mods[j].value >= FP_MAX_IN : !wide && mods[j].value > 4 * m.value;
         c.in = src + (size_t)cb * sstride + ((size_t)j << logn);
         c.out = digits + ((((size_t)cb * L + j) * (L + 1) + i) << logn);
         return c;
@@ -280,6 +293,7 @@ struct SpecialInttOp {
     __device__ Ctx ctx(int b) const {
         Ctx c;
         c.lm = make_limb(mods[K - 1], 0);
+        c.lm.fp = fp_form(mods[K - 1]);
         c.in = acc + (((size_t)b * (L + 1) + L) << logn);
         c.out = last + ((size_t)b << logn);
         return c;
@@ -328,6 +342,7 @@ struct SpecialInnerOp {
         c.d = digits + (((size_t)cb * L * (L + 1) + L) << logn);
         c.k = keys.of((uint32_t)cb) + (((size_t)comp * K + K - 1) << logn);
         c.out = last + ((size_t)b << logn);
+        c.lm.fp = fp_form(m);
         c.islack = 1;
         return c;
     }
@@ -367,6 +382,7 @@ struct ModDownBase {
     const Mod *mods;
     const DropC *drop;        // row for the special prime: drop[K*K + j]
     int L, K, logn;
+    int B;                    // ciphertexts of the launch
     struct Ctx {
         NttLimb lm;
         const uint64_t *acc;
@@ -380,7 +396,7 @@ struct ModDownBase {
     };
     static constexpr bool wide_slack = true;
     __device__ Ctx make(int b) const {
-        const int j = b % L, bc = b / L;  // bc = cb*2 + c
+        const int j = b / (2 * B), bc = b % (2 * B);  // modulus by modulus; bc = cb*2 + c
         const int cb = bc >> 1, cc = bc & 1;
         const Mod &m = mods[j];
         Ctx c;
@@ -388,7 +404,9 @@ struct ModDownBase {
         c.ratio_hi = m.ratio_hi;
         c.d = drop[(size_t)K * K + j];
         c.reduce = mods[K - 1].value > m.value;
-        c.slack = (logn <= MAX_LOGB && m.value < (1ull << 57)) ? SLACK_WIDE : m.value < (1ull << 60) ? SLACK_M : 0;
+        c.lm.fp = fp_form(m);
+        c.slack = c.lm.fp ? 0 : (logn <= MAX_LOGB && m.value < (1ull << 57)) ? SLACK_WIDE
+                              : m.value < (1ull << 60) ? SLACK_M : 0;
         c.wide_off = (m.ratio_hi - 1) * m.value;
         c.acc = acc + (((size_t)bc * (L + 1) + j) << logn);
         c.last = last + ((size_t)bc << logn);
@@ -541,7 +559,7 @@ int keyswitch_groups(const Context &c, int L, const uint64_t *target, uint64_t t
             e = dispatch_ntt<false>(logn, op, (unsigned)(nb * L), logn, 1, s);
             if (e != cudaSuccess) return status_from(e);
         }
-        ModUpOp mu{ckks ? tgt : tg, ckks ? (uint64_t)L * n : tstride, digits, c.d_mods, nullptr, L, K, ckks, logn};
+        ModUpOp mu{ckks ? tgt : tg, ckks ? (uint64_t)L * n : tstride, digits, c.d_mods, nullptr, L, K, ckks, logn, (int)nb};
         {
             TraceScope ts("ks_modup_ntt", s);
             e = dispatch_ntt<true>(logn, mu, (unsigned)(nb * pairs), 0, 0, s);
@@ -563,7 +581,7 @@ int keyswitch_groups(const Context &c, int L, const uint64_t *target, uint64_t t
             e = dispatch_ntt<false>(logn, si, (unsigned)(nb * 2), logn, 1, s);
         }
         if (e != cudaSuccess) return status_from(e);
-        ModDownBase mb{acc, last, cc, cstride, c.d_mods, c.d_drop, L, K, logn};
+        ModDownBase mb{acc, last, cc, cstride, c.d_mods, c.d_drop, L, K, logn, (int)nb};
         TraceScope ts("ks_moddown", s);
         if (ckks) {
             ModDownCkksOp op{mb};
@@ -664,7 +682,7 @@ int keyswitch_shapes(const KsShape *shapes, int count, cudaStream_t s) {
             const uint64_t tstride = sh.tstride ? sh.tstride : (uint64_t)sh.L * sh.c->n;
             t.op[t.count] = ModUpOp{ckks ? buf[k].tgt : sh.target, ckks ? (uint64_t)sh.L * sh.c->n : tstride,
                                     buf[k].digits, sh.c->d_mods, nullptr, sh.L, (int)sh.c->chain.size(), ckks ? 1 : 0,
-                                    sh.c->logn};
+                                    sh.c->logn, (int)sh.B};
             t.logn[t.count] = sh.c->logn;
             t.first[t.count] = f;
             f += (unsigned)(sh.B * (ckks ? sh.L * sh.L : sh.L * (sh.L + 1)));
@@ -733,7 +751,7 @@ int keyswitch_shapes(const KsShape *shapes, int count, cudaStream_t s) {
         const Context &c = *sh.c;
         const int K = (int)c.chain.size();
         const uint64_t cstride = sh.cstride ? sh.cstride : 2ull * sh.L * c.n;
-        const ModDownBase mb{buf[k].acc, buf[k].last, sh.ct, cstride, c.d_mods, c.d_drop, sh.L, K, c.logn};
+        const ModDownBase mb{buf[k].acc, buf[k].last, sh.ct, cstride, c.d_mods, c.d_drop, sh.L, K, c.logn, (int)sh.B};
         const unsigned limbs = (unsigned)(sh.B * 2 * sh.L);
         if (c.scheme == SCHEME_CKKS) {
             tc.op[tc.count] = ModDownCkksOp{mb};
@@ -1088,7 +1106,7 @@ int relinearize_noalloc(const Context &c, int L, uint64_t *ct3, uint64_t cstride
             e = dispatch_ntt<false>(logn, op, (unsigned)(nb * L), logn, 1, s);
             if (e != cudaSuccess) return status_from(e);
         }
-        ModUpOp mu{ckks ? tgt : tg, ckks ? (uint64_t)L * n : tstride, digits, c.d_mods, nullptr, L, K, ckks, logn};
+        ModUpOp mu{ckks ? tgt : tg, ckks ? (uint64_t)L * n : tstride, digits, c.d_mods, nullptr, L, K, ckks, logn, (int)nb};
         e = dispatch_ntt<true>(logn, mu, (unsigned)(nb * pairs), 0, 0, s);
         if (e != cudaSuccess) return status_from(e);
         const int threads = 128;
@@ -1099,7 +1117,7 @@ int relinearize_noalloc(const Context &c, int L, uint64_t *ct3, uint64_t cstride
         SpecialInttOp si{acc, last, c.d_mods, L, K, c.scheme == SCHEME_BGV, logn};
         e = dispatch_ntt<false>(logn, si, (unsigned)(nb * 2), logn, 1, s);
         if (e != cudaSuccess) return status_from(e);
-        ModDownBase mb{acc, last, cc, cstride, c.d_mods, c.d_drop, L, K, logn};
+        ModDownBase mb{acc, last, cc, cstride, c.d_mods, c.d_drop, L, K, logn, (int)nb};
         if (ckks) {
             ModDownCkksOp op{mb};
             e = dispatch_ntt<true>(logn, op, (unsigned)(nb * 2 * L), 0, 0, s);

@@ -357,6 +357,7 @@ struct PackedNttOp {
     __device__ Ctx ctx(int b) const {
         Ctx c;
         c.lm = make_limb(mods[b % limbs], 0);
+        c.lm.fp = fp_form(mods[b % limbs]);
         c.in = in + ((size_t)b << logn);
         c.out = out + ((size_t)b << logn);
         return c;
@@ -392,6 +393,7 @@ struct PairNttOp {
         const int ct = p >> 2, slot = p & 3;
         Ctx c;
         c.lm = make_limb(mods[l], 0);
+        c.lm.fp = fp_form(mods[l]);
         c.in = (slot < 2 ? a + (size_t)ct * astride + (((size_t)slot * L + l) << logn)
                          : b + (size_t)ct * bstride + (((size_t)(slot - 2) * L + l) << logn));
         c.out = out + ((size_t)blk << logn);
@@ -421,6 +423,7 @@ struct CtInttOutOp {
         const int p = b / L;
         Ctx c;
         c.lm = make_limb(mods[l], 0);
+        c.lm.fp = fp_form(mods[l]);
         c.in = in + ((size_t)b << logn);
         c.out = out + (size_t)(p / per) * ostride + (((size_t)(p % per) * L + l) << logn);
         return c;

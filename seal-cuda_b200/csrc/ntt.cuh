@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "fp64mod.cuh"
 
 namespace tb {
 
@@ -38,7 +39,14 @@ struct NttLimb {
     uint64_t inv_n, inv_n_quo;   // N^-1 (Shoup)
     uint64_t sroot, sroot_quo;   // last inverse root times N^-1 (Shoup)
     uint32_t sb;                 // sub-block index when the CTA owns 2^LOGB of a longer limb
+    // FP64 form (fp64mod.cuh), 0 = integer form: FP_ON, with FP_RED for moduli of 2^48 and
+    // above (values reduced at every pass) and FP_RED_IN where the inputs may exceed q
+    // (inverse transforms: reduced as they are loaded)
+    int fp;
+    const FpMod *fpm;
 };
+
+enum { FP_ON = 1, FP_RED = 2, FP_RED_IN = 4 };
 
 // Threads per CTA: variant 0 gives each thread one radix-8 group per pass at a time (at
 // most 1024 threads); variant V >= 1 divides the thread count by 2^V, each thread then
@@ -58,11 +66,17 @@ struct NttCfg {
     static constexpr int BASE = NB >= 8192 ? 1024 : (NB / 8 >= 64 ? NB / 8 : 64);
     static constexpr int THREADS = (BASE >> V) >= 32 ? (BASE >> V) : 32;
     static constexpr int REM = LOGB % 3;
+    // CTAs per SM the registers are held to: 1024 threads at 64 registers, as far as the
+    // shared memory allows (227 KB per SM). Unbounded, the 512-thread kernels of 2^13
+    // limbs took more than 64 and ran one CTA per SM (a BGV mod-up 88 us instead of 76).
+    static constexpr int BY_SMEM = (227 * 1024) / (8 * NB) > 0 ? (227 * 1024) / (8 * NB) : 1;
+    static constexpr int BY_REGS = 1024 / THREADS < 8 ? 1024 / THREADS : 8;
+    static constexpr int CTAS = BY_SMEM < BY_REGS ? BY_SMEM : BY_REGS;
 };
 
 // Shared-memory slot of coefficient base | (k << logsub) when the bits of k << logsub
 // are clear in base: swz(base) ^ swz_delta(k << logsub), a compile-time constant per k.
-__host__ __device__ constexpr int swz_delta(int kk) { return kk ^ ((kk >> 4) & 15); }
+__host__ __device__ constexpr int swz_delta(int kk) { return swz(kk); }
 
 __device__ __forceinline__ void ct_butterfly(uint64_t &x, uint64_t &y, ulonglong2 w, uint64_t q, uint64_t q2) {
     uint64_t u = csub(x, q2);
@@ -287,6 +301,130 @@ __device__ __forceinline__ void fwd_passes(const Op &op, const Ctx &c, uint64_t 
     }
 }
 
+// ---------------------------------------------------------------- FP64 form, forward
+// The same passes with exact FP64 arithmetic (fp64mod.cuh) for moduli below 2^50, used by
+// one-CTA and CTA-pair limbs of 2^12 .. 2^15 coefficients whose stores take canonical
+// outputs. Without any reduction a value grows by at most q (1/2 + 2^-53 B) a stage from
+// the bound B so far: for q < 2^48 and inputs below 4 q (or below 2^49) it stays below
+// 2^52 through 15 stages; for q < 2^50 every pass first reduces its values to q/2, and
+// three stages add less than 2 q. The copy-out reduces to [0, q).
+//
+// What bounds it: shared-memory wavefronts and the FP64 pipe, both busy 55 - 65% of the
+// cycles (the integer form: the FMA-heavy pipe). Measured, 2048 limbs of 2^14 modulo 40-bit
+// primes, each input read by 8 limbs: 0.197 ms against 0.312 ms of the wide integer form.
+// In a pass whose strides are below 32 every lane group has twiddles of its own: there the
+// twiddles alone are loaded (8 bytes, side by side across the warp, before the data) and
+// the quotients multiplied out, half the table traffic: 4% faster than loading pairs. The
+// other passes share twiddles across the warp and load pairs. One loop over the passes
+// with the stage as a variable, instead of a copy of the code each, was 6% slower and no
+// faster for a single transform.
+struct FpPass {
+    const double *w;    // twiddles
+    const double2 *p;   // {twiddle, quotient}
+    double q, qinv;
+    bool red;           // reduce the pass's inputs
+};
+
+// R_LOG Cooley-Tukey stages on R values; tw(t, k) gives twiddle k (stage t) and quotient.
+template <int R_LOG, class Tw>
+__device__ __forceinline__ void fwd_group_fp(double (&v)[1 << R_LOG], const Tw &tw, const FpPass &f) {
+    constexpr int R = 1 << R_LOG;
+    if (f.red) {
+#pragma unroll
+        for (int k = 0; k < R; k++) v[k] = fp_reduce(v[k], f.q, f.qinv);
+    }
+#pragma unroll
+    for (int t = 0; t < R_LOG; t++) {
+        const int half = R >> (t + 1);
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            if (k & half) continue;
+            const double2 m = tw(t, (1 << t) - 1 + (k >> (R_LOG - t)));
+            const double r = fp_mulmod(v[k + half], m.x, m.y, f.q);
+            v[k + half] = __dadd_rn(v[k], -r);
+            v[k] = __dadd_rn(v[k], r);
+        }
+    }
+}
+
+// Pass of R_LOG stages starting at local stage s (compare fwd_pass). The remainder pass's
+// twiddles are in natural order.
+// S0: the global stage of local stage 0.
+template <int R_LOG, bool FROM_GLOBAL, int LOGB, int T, int s, int S0, class Op, class Ctx>
+__device__ __forceinline__ void fwd_pass_fp(const Op &op, const Ctx &c, double *sm, const FpPass &f) {
+    constexpr int R = 1 << R_LOG, NB = 1 << LOGB, G = NB >> R_LOG, IT = (G + T - 1) / T;
+    constexpr int logsub = LOGB - s - R_LOG;
+    constexpr bool OWN = R_LOG == 3 && logsub < 5;
+    constexpr int gs = S0 + s;   // global stage of this pass
+#pragma unroll
+    for (int i = 0; i < IT; i++) {
+        const int g = pass_group<!FROM_GLOBAL, T, IT>(i);
+        if (G % T != 0 && g >= G) continue;
+        const int base = ((g >> logsub) << (LOGB - s)) + (g & ((1 << logsub) - 1));
+        const int sb = swz(base);
+        const uint32_t X = (1u << gs) + (c.lm.sb << s) + (uint32_t)(g >> logsub);
+        double w[R];
+        if constexpr (OWN) {
+            const double *row = f.w + X;
+#pragma unroll
+            for (int k = 0; k < R - 1; k++) w[k] = __ldg(row + (k << gs));
+        }
+        const double2 *prow = f.p + X;
+        double v[R];
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            if constexpr (FROM_GLOBAL) v[k] = fp_from_u64(op.load(c, base + (k << logsub)));
+            else v[k] = sm[sb ^ swz_delta(k << logsub)];
+        }
+        fwd_group_fp<R_LOG>(
+            v,
+            [&](int t, int k) {
+                if constexpr (OWN) return make_double2(w[k], __dmul_rn(w[k], f.qinv));
+                else if constexpr (R_LOG == 3) return __ldg(prow + (k << gs));
+                else return __ldg(f.p + ((X << t) + (uint32_t)(k - ((1 << t) - 1))));
+            },
+            f);
+#pragma unroll
+        for (int k = 0; k < R; k++) sm[sb ^ swz_delta(k << logsub)] = v[k];
+    }
+    // warp barriers as in fwd_pass
+    constexpr int LIT = (IT > 1 && T % 32 == 0) ? ilog2c<IT>() : 0;
+    if constexpr (!FROM_GLOBAL && R_LOG == 3 && logsub >= 3 && logsub <= 5 + LIT && T % 32 == 0) __syncwarp();
+    else if constexpr (!FROM_GLOBAL && R_LOG == 3 && logsub == 0 && WarpIO<NB, T>::value) __syncwarp();
+    else __syncthreads();
+}
+
+template <int S, int LOGB, int T, int S0, class Op, class Ctx>
+__device__ __forceinline__ void fwd_passes_fp(const Op &op, const Ctx &c, double *sm, const FpPass &f) {
+    if constexpr (S < LOGB) {
+        fwd_pass_fp<3, false, LOGB, T, S, S0>(op, c, sm, f);
+        fwd_passes_fp<S + 3, LOGB, T, S0>(op, c, sm, f);
+    }
+}
+
+template <int LOGB, int T, int S0, bool FROM_GLOBAL, class Op, class Ctx>
+__device__ __forceinline__ void ntt_fwd_block_fp(const Op &op, const Ctx &c, double *sm, const FpPass &f) {
+    constexpr int FIRST = LOGB % 3 != 0 ? LOGB % 3 : 3;
+    fwd_pass_fp<FIRST, FROM_GLOBAL, LOGB, T, 0, S0>(op, c, sm, f);
+    fwd_passes_fp<FIRST, LOGB, T, S0>(op, c, sm, f);
+}
+
+// FP64 values in shared memory to canonical words in the same slots' order for the
+// copy-out of fwd_copy_out.
+struct FpWords {
+    const double *sm;
+    double q, qinv;
+    uint64_t qi;
+    __device__ __forceinline__ ulonglong2 pair(int p) const {
+        const double2 w = *reinterpret_cast<const double2 *>(&sm[p & ~1]);
+        return make_ulonglong2(fp_to_residue(fp_reduce(w.x, q, qinv), qi), fp_to_residue(fp_reduce(w.y, q, qinv), qi));
+    }
+};
+struct IntWords {
+    const uint64_t *sm;
+    __device__ __forceinline__ ulonglong2 pair(int p) const { return *reinterpret_cast<const ulonglong2 *>(&sm[p & ~1]); }
+};
+
 // Copy-out of a forward transform: coefficient pairs (e, e+1) from shared memory to
 // op.store2. An Op whose epilogue reads global memory declares `Epi` with
 // epi2(ctx, e) (the reads for a pair) and store2(ctx, e, a, b, epi): the reads of
@@ -297,15 +435,15 @@ struct HasEpi : std::false_type {};
 template <class Op>
 struct HasEpi<Op, std::void_t<typename Op::Epi>> : std::true_type {};
 
-template <int NB, int T, class Op, class Ctx>
-__device__ __forceinline__ void fwd_copy_out(const Op &op, const Ctx &c, const uint64_t *sm, int off) {
+template <int NB, int T, class Words, class Op, class Ctx>
+__device__ __forceinline__ void fwd_copy_out_words(const Op &op, const Ctx &c, const Words &words, int off) {
     constexpr int ITER = NB / (2 * T);
     if constexpr (WarpIO<NB, T>::value && !HasEpi<Op>::value) {
 #pragma unroll
         for (int i = 0; i < ITER; i++) {
             const int e = io_pair<NB, T>(i);
             const int p = swz(e);
-            const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(&sm[p & ~1]);
+            const ulonglong2 w = words.pair(p);
             // a select, not a branch: the slot parity changes every 8 lanes, and a branch
             // would run both copies of the store (and its reductions) one after the other
             const uint64_t a = (p & 1) ? w.y : w.x, b = (p & 1) ? w.x : w.y;
@@ -323,7 +461,7 @@ __device__ __forceinline__ void fwd_copy_out(const Op &op, const Ctx &c, const u
             for (int i = 0; i < BATCH; i++) {
                 const int e = io_pair<NB, T>(i0 + i);
                 const int p = swz(e);
-                const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(&sm[p & ~1]);
+                const ulonglong2 w = words.pair(p);
                 const uint64_t a = (p & 1) ? w.y : w.x, b = (p & 1) ? w.x : w.y;
                 op.store2(c, e + off, a, b, pre[i]);
             }
@@ -331,12 +469,22 @@ __device__ __forceinline__ void fwd_copy_out(const Op &op, const Ctx &c, const u
     } else {
         for (int e = threadIdx.x * 2; e < NB; e += T * 2) {
             const int p = swz(e);
-            const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(&sm[p & ~1]);
+            const ulonglong2 w = words.pair(p);
             const uint64_t a = (p & 1) ? w.y : w.x, b = (p & 1) ? w.x : w.y;
             if constexpr (HasEpi<Op>::value) op.store2(c, e + off, a, b, op.epi2(c, e + off));
             else op.store2(c, e + off, a, b);
         }
     }
+}
+
+template <int NB, int T, class Op, class Ctx>
+__device__ __forceinline__ void fwd_copy_out(const Op &op, const Ctx &c, const uint64_t *sm, int off) {
+    fwd_copy_out_words<NB, T>(op, c, IntWords{sm}, off);
+}
+
+template <int NB, int T, class Op, class Ctx>
+__device__ __forceinline__ void fwd_copy_out_fp(const Op &op, const Ctx &c, const double *sm, int off) {
+    fwd_copy_out_words<NB, T>(op, c, FpWords{sm, c.lm.fpm->q, c.lm.fpm->qinv, c.lm.q}, off);
 }
 
 // One limb (or sub-block) b of Op by a CTA of T threads, starting at global stage s0.
@@ -349,10 +497,22 @@ __device__ __forceinline__ void ntt_fwd_block(const Op &op, const Ctx &c, uint64
     fwd_copy_out<1 << LOGB, T>(op, c, sm, 0);   // coalesced, two coefficients per thread
 }
 
+constexpr int FP_MIN_LOGN = 12;   // degrees with FP64 forms: 2^12 .. 2^15
+constexpr int FP_MAX_LOGN = 15;
+
 template <int LOGB, int T, class Op>
 __device__ __forceinline__ void ntt_fwd_limb(const Op &op, int limb, int s0, uint64_t *sm) {
     const auto c = op.ctx(limb);
     const uint32_t rbase = (1u << s0) + c.lm.sb;
+    if constexpr (LOGB >= FP_MIN_LOGN) {
+        if (c.lm.fp && s0 == 0) {
+            double *smd = reinterpret_cast<double *>(sm);
+            const FpPass f{c.lm.fpm->w, c.lm.fpm->p, c.lm.fpm->q, c.lm.fpm->qinv, (c.lm.fp & FP_RED) != 0};
+            ntt_fwd_block_fp<LOGB, T, 0, true>(op, c, smd, f);
+            fwd_copy_out_fp<1 << LOGB, T>(op, c, smd, 0);
+            return;
+        }
+    }
     if constexpr (HasSlack<decltype(c)>::value) {
         if constexpr (WideSlack<Op>::value) {
             if (c.slack == SLACK_WIDE) {
@@ -369,7 +529,7 @@ __device__ __forceinline__ void ntt_fwd_limb(const Op &op, int limb, int s0, uin
 }
 
 template <int LOGB, int V, class Op>
-__global__ void __launch_bounds__(NttCfg<LOGB, V>::THREADS) ntt_fwd_kernel(Op op, int s0) {
+__global__ void __launch_bounds__(NttCfg<LOGB, V>::THREADS, NttCfg<LOGB, V>::CTAS) ntt_fwd_kernel(Op op, int s0) {
     extern __shared__ uint64_t sm[];
     ntt_fwd_limb<LOGB, NttCfg<LOGB, V>::THREADS>(op, blockIdx.x, s0, sm);
 }
@@ -467,32 +627,129 @@ __device__ __forceinline__ void inv_passes(const Op &op, const Ctx &c, uint64_t 
     }
 }
 
+// ---------------------------------------------------------------- FP64 form, inverse
+// Gentleman-Sande passes in exact FP64 arithmetic (see the forward form). A sum doubles
+// the bound, a product brings it back to about q/2, so of a radix-8 group's outputs the
+// first two are reduced (the other six pass through a product in the last two stages):
+// in units of q, inputs below 1.34 give differences below 10.7 (16 is the limit for
+// q < 2^48) and outputs below 1.34. For q < 2^50 (limit 4) every pass reduces its inputs,
+// and the sums of four before the last stage. The scaled last stage multiplies both of
+// its outputs, so the store gets |x| < q. Inputs are below q, or reduced as they are
+// loaded (FP_RED_IN).
+// Pass of R_LOG stages starting at stage s (compare inv_pass).
+template <int R_LOG, bool TO_GLOBAL, bool SCALE, int LOGB, int T, int s, int LOGN, class Op, class Ctx>
+__device__ __forceinline__ void inv_pass_fp(const Op &op, const Ctx &c, double *sm, const FpPass &f) {
+    constexpr int R = 1 << R_LOG, NB = 1 << LOGB, G = NB >> R_LOG, IT = (G + T - 1) / T;
+    constexpr bool OWN = R_LOG == 3 && s < 5;
+    const double q = f.q, qinv = f.qinv;
+    constexpr uint32_t n = 1u << LOGN, skip = n - (n >> 4);
+    const double si = SCALE ? c.lm.fpm->inv_n : 0.0, sr = SCALE ? c.lm.fpm->sroot : 0.0;
+    const uint64_t qi = c.lm.q;
+#pragma unroll
+    for (int i = 0; i < IT; i++) {
+        const int g = pass_group<true, T, IT>(i);
+        if (G % T != 0 && g >= G) continue;
+        const int base = ((g >> s) << (s + R_LOG)) + (g & ((1 << s) - 1));
+        const int sb = swz(base);
+        const uint32_t blk = (c.lm.sb << (LOGB - s - R_LOG)) + (uint32_t)(g >> s);
+        // radix 8: twiddle k (4, 2, 1 of the three stages); else stages in natural order
+        auto at = [&](int t, int k) -> uint32_t {
+            if constexpr (R_LOG == 3) return n + 1 - (n >> s) + (uint32_t)k * (n >> (s + 3)) + blk;
+            else if constexpr (R_LOG == 2) return t == 0 ? n + 1 - (n >> s) + 2 * blk + (uint32_t)k : n + 1 - (n >> (s + 1)) + blk;
+            else return n + 1 - (n >> s) + blk;
+        };
+        double w[R];
+        if constexpr (OWN) {
+#pragma unroll
+            for (int k = 0; k < R - 1; k++) w[k] = __ldg(f.w + blk + (n + 1 - (n >> s) + (uint32_t)k * (n >> (s + 3))));
+        }
+        double v[R];
+#pragma unroll
+        for (int k = 0; k < R; k++) v[k] = sm[sb ^ swz_delta(k << s)];
+        if (f.red) {
+#pragma unroll
+            for (int k = 0; k < R; k++) v[k] = fp_reduce(v[k], q, qinv);
+        }
+#pragma unroll
+        for (int t = 0; t < R_LOG; t++) {
+            const int h = 1 << t;
+            if (R_LOG == 3 && t == 2 && f.red) {
+                v[0] = fp_reduce(v[0], q, qinv);
+                v[4] = fp_reduce(v[4], q, qinv);
+            }
+#pragma unroll
+            for (int k = 0; k < R; k++) {
+                if (k & h) continue;
+                const double x = v[k], y = v[k + h];
+                if (SCALE && t == R_LOG - 1) {
+                    v[k] = fp_mulmod(__dadd_rn(x, y), si, __dmul_rn(si, qinv), q);
+                    v[k + h] = fp_mulmod(__dadd_rn(x, -y), sr, __dmul_rn(sr, qinv), q);
+                } else {
+                    const int ki = R - (R >> t) + (k >> (t + 1));
+                    const double2 m = OWN ? make_double2(w[ki], __dmul_rn(w[ki], qinv)) : (R_LOG == 3 ? __ldg(f.p + blk + (n + 1 - (n >> s) - skip + (uint32_t)ki * (n >> (s + 3)))) : __ldg(f.p + (at(t, ki) - skip)));
+                    v[k] = __dadd_rn(x, y);
+                    v[k + h] = fp_mulmod(__dadd_rn(x, -y), m.x, m.y, q);
+                }
+            }
+        }
+        if constexpr (!SCALE && R_LOG >= 2) {
+            v[0] = fp_reduce(v[0], q, qinv);
+            if constexpr (R_LOG == 3) v[1] = fp_reduce(v[1], q, qinv);
+        }
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            if constexpr (TO_GLOBAL) op.store(c, base + (k << s), fp_to_residue(v[k], qi));
+            else sm[sb ^ swz_delta(k << s)] = v[k];
+        }
+    }
+    // warp barriers as in inv_pass
+    if constexpr (!TO_GLOBAL) {
+        constexpr int LIT = (IT > 1 && T % 32 == 0) ? ilog2c<IT>() : 0;
+        constexpr int PASSES_8 = (LOGB % 3) ? LOGB / 3 : LOGB / 3 - 1;
+        if constexpr (R_LOG == 3 && s + 3 < 3 * PASSES_8 && s + 3 <= 5 + LIT && T % 32 == 0) __syncwarp();
+        else __syncthreads();
+    }
+}
+
+template <int P, int PASSES, int LOGB, int T, int LOGN, class Op, class Ctx>
+__device__ __forceinline__ void inv_passes_fp(const Op &op, const Ctx &c, double *sm, const FpPass &f) {
+    if constexpr (P < PASSES) {
+        inv_pass_fp<3, false, false, LOGB, T, 3 * P, LOGN>(op, c, sm, f);
+        inv_passes_fp<P + 1, PASSES, LOGB, T, LOGN>(op, c, sm, f);
+    }
+}
+
 // Copy-in of an inverse transform: coefficient pairs from op.load2 (coefficient e + off)
 // into shared memory, then the barrier before the first pass: a warp barrier when the
 // copy-in is warp-major and the first pass is a radix-8 pass (each warp then reads
 // exactly what it wrote), a CTA barrier otherwise.
-template <int LOGB, int T, class Op, class Ctx>
+// FP: the words become doubles (reduced with FP_RED_IN), in the same slots.
+template <int LOGB, int T, bool FP = false, class Op, class Ctx>
 __device__ __forceinline__ void inv_copy_in(const Op &op, const Ctx &c, uint64_t *sm, int off) {
     constexpr int NB = 1 << LOGB;
     constexpr int PASSES_8 = (LOGB % 3) ? LOGB / 3 : LOGB / 3 - 1;
-    if constexpr (WarpIO<NB, T>::value) {
-#pragma unroll 4
-        for (int i = 0; i < NB / (2 * T); i++) {
-            const int e = io_pair<NB, T>(i);
-            uint64_t a, b;
-            op.load2(c, e + off, a, b);
-            const int p = swz(e);
+    auto put = [&](int e) {
+        uint64_t a, b;
+        op.load2(c, e + off, a, b);
+        const int p = swz(e);
+        if constexpr (FP) {
+            double x = fp_from_u64(a), y = fp_from_u64(b);
+            if (c.lm.fp & FP_RED_IN) {
+                x = fp_reduce(x, c.lm.fpm->q, c.lm.fpm->qinv);
+                y = fp_reduce(y, c.lm.fpm->q, c.lm.fpm->qinv);
+            }
+            *reinterpret_cast<double2 *>(&sm[p & ~1]) = (p & 1) ? make_double2(y, x) : make_double2(x, y);
+        } else {
             *reinterpret_cast<ulonglong2 *>(&sm[p & ~1]) = (p & 1) ? make_ulonglong2(b, a) : make_ulonglong2(a, b);
         }
+    };
+    if constexpr (WarpIO<NB, T>::value) {
+#pragma unroll 4
+        for (int i = 0; i < NB / (2 * T); i++) put(io_pair<NB, T>(i));
         if constexpr (PASSES_8 >= 1) __syncwarp();
         else __syncthreads();
     } else {
-        for (int e = threadIdx.x * 2; e < NB; e += T * 2) {
-            uint64_t a, b;
-            op.load2(c, e + off, a, b);
-            const int p = swz(e);
-            *reinterpret_cast<ulonglong2 *>(&sm[p & ~1]) = (p & 1) ? make_ulonglong2(b, a) : make_ulonglong2(a, b);
-        }
+        for (int e = threadIdx.x * 2; e < NB; e += T * 2) put(e);
         __syncthreads();
     }
 }
@@ -501,16 +758,25 @@ __device__ __forceinline__ void inv_copy_in(const Op &op, const Ctx &c, uint64_t
 // stage is the transform's last stage (whole limb).
 template <int LOGB, int T, class Op>
 __device__ __forceinline__ void ntt_inv_limb(const Op &op, int limb, int logn, int scale_last, uint64_t *sm) {
-    constexpr int NB = 1 << LOGB;
     constexpr int REM = LOGB % 3;
     const auto c = op.ctx(limb);
-    inv_copy_in<LOGB, T>(op, c, sm, 0);
     constexpr int LAST = REM ? REM : 3;
     constexpr int PASSES = REM ? LOGB / 3 : LOGB / 3 - 1;  // radix-8 passes before the last one
+    if constexpr (LOGB >= FP_MIN_LOGN) {
+        if (c.lm.fp && scale_last) {
+            double *smd = reinterpret_cast<double *>(sm);
+            const FpPass f{c.lm.fpm->iw, c.lm.fpm->ip, c.lm.fpm->q, c.lm.fpm->qinv, (c.lm.fp & FP_RED) != 0};
+            inv_copy_in<LOGB, T, true>(op, c, sm, 0);
+            inv_passes_fp<0, PASSES, LOGB, T, LOGB>(op, c, smd, f);
+            inv_pass_fp<LAST, true, true, LOGB, T, 3 * PASSES, LOGB>(op, c, smd, f);
+            return;
+        }
+    }
+    inv_copy_in<LOGB, T>(op, c, sm, 0);
     if constexpr (HasInvSlack<decltype(c)>::value) {
-        if (c.islack && scale_last) {
-            inv_passes<0, PASSES, LOGB, T, false, true>(op, c, sm, logn);
-            inv_pass<LAST, true, true, LOGB, T, 3 * PASSES, false, true>(op, c, sm, logn);
+        if (c.islack && scale_last) {   // a whole limb: constant table offsets
+            inv_passes<0, PASSES, LOGB, T, false, true>(op, c, sm, LOGB);
+            inv_pass<LAST, true, true, LOGB, T, 3 * PASSES, false, true>(op, c, sm, LOGB);
             return;
         }
     }
@@ -520,7 +786,7 @@ __device__ __forceinline__ void ntt_inv_limb(const Op &op, int limb, int logn, i
 }
 
 template <int LOGB, int V, class Op>
-__global__ void __launch_bounds__(NttCfg<LOGB, V>::THREADS) ntt_inv_kernel(Op op, int logn, int scale_last) {
+__global__ void __launch_bounds__(NttCfg<LOGB, V>::THREADS, NttCfg<LOGB, V>::CTAS) ntt_inv_kernel(Op op, int logn, int scale_last) {
     extern __shared__ uint64_t sm[];
     ntt_inv_limb<LOGB, NttCfg<LOGB, V>::THREADS>(op, blockIdx.x, logn, scale_last, sm);
 }
@@ -538,7 +804,7 @@ __global__ void __launch_bounds__(NttCfg<LOGB, V>::THREADS) ntt_inv_kernel(Op op
 // transform, and the Op's load / store see whole-limb coefficient indices, so every
 // fused operation works at this length unchanged.
 template <int LOGB, int V, class Op>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NttCfg<LOGB, V>::THREADS)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NttCfg<LOGB, V>::THREADS, NttCfg<LOGB, V>::CTAS)
     ntt_fwd_pair_kernel(Op op) {
     extern __shared__ uint64_t sm[];
     constexpr int NB = 1 << LOGB;
@@ -548,6 +814,28 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NttCfg<LOGB, V>::THR
     const unsigned half = cl.block_rank();
     auto c = op.ctx((int)(blockIdx.x >> 1));
     c.lm.sb = half;
+    if constexpr (LOGB + 1 >= FP_MIN_LOGN) {
+        if (c.lm.fp) {
+            double *smd = reinterpret_cast<double *>(sm);
+            const FpPass f{c.lm.fpm->w, c.lm.fpm->p, c.lm.fpm->q, c.lm.fpm->qinv, (c.lm.fp & FP_RED) != 0};
+            const double w = __ldg(f.w + 1), wq = __dmul_rn(w, f.qinv);
+#pragma unroll 2
+            for (int j = threadIdx.x; j < NB; j += T) {
+                double x = fp_from_u64(op.load(c, j)), y = fp_from_u64(op.load(c, j + NB));
+                if (f.red) {
+                    x = fp_reduce(x, f.q, f.qinv);
+                    y = fp_reduce(y, f.q, f.qinv);
+                }
+                const double r = fp_mulmod(y, w, wq, f.q);
+                smd[swz(j)] = half ? __dadd_rn(x, -r) : __dadd_rn(x, r);
+            }
+            __syncthreads();
+            ntt_fwd_block_fp<LOGB, T, 1, false>(op, c, smd, f);
+            cl.sync();   // both CTAs have read every input coefficient
+            fwd_copy_out_fp<NB, T>(op, c, smd, (int)half << LOGB);
+            return;
+        }
+    }
     {
         const uint64_t q = c.lm.q, q2 = q << 1;
         const ulonglong2 w = __ldg(c.lm.roots + 1);
@@ -567,7 +855,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NttCfg<LOGB, V>::THR
 }
 
 template <int LOGB, int V, class Op>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NttCfg<LOGB, V>::THREADS)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NttCfg<LOGB, V>::THREADS, NttCfg<LOGB, V>::CTAS)
     ntt_inv_pair_kernel(Op op) {
     namespace cg = cooperative_groups;
     extern __shared__ uint64_t sm[];
@@ -579,9 +867,36 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NttCfg<LOGB, V>::THR
     auto c = op.ctx((int)(blockIdx.x >> 1));
     c.lm.sb = half;
     const int off = (int)half << LOGB;
-    inv_copy_in<LOGB, T>(op, c, sm, off);
     constexpr int LAST = REM ? REM : 3;
     constexpr int PASSES = REM ? LOGB / 3 : LOGB / 3 - 1;
+    if constexpr (LOGB + 1 >= FP_MIN_LOGN) {
+        if (c.lm.fp) {
+            double *smd = reinterpret_cast<double *>(sm);
+            const FpPass f{c.lm.fpm->iw, c.lm.fpm->ip, c.lm.fpm->q, c.lm.fpm->qinv, (c.lm.fp & FP_RED) != 0};
+            inv_copy_in<LOGB, T, true>(op, c, sm, off);
+            inv_passes_fp<0, PASSES, LOGB, T, LOGB + 1>(op, c, smd, f);
+            inv_pass_fp<LAST, false, false, LOGB, T, 3 * PASSES, LOGB + 1>(op, c, smd, f);
+            cl.sync();
+            // the scaled last stage: this CTA's outputs from both halves
+            const double *lo = cl.map_shared_rank(smd, 0u), *hi = cl.map_shared_rank(smd, 1u);
+            const double sc = half ? c.lm.fpm->sroot : c.lm.fpm->inv_n;
+            const double scq = __dmul_rn(sc, f.qinv);
+#pragma unroll 2
+            for (int j = threadIdx.x; j < NB; j += T) {
+                const int p = swz(j);
+                double x = lo[p], y = hi[p];
+                if (f.red) {
+                    x = fp_reduce(x, f.q, f.qinv);
+                    y = fp_reduce(y, f.q, f.qinv);
+                }
+                const double v = fp_mulmod(half ? __dadd_rn(x, -y) : __dadd_rn(x, y), sc, scq, f.q);
+                op.store(c, j + off, fp_to_residue(v, c.lm.q));
+            }
+            cl.sync();   // the partner has read this CTA's half
+            return;
+        }
+    }
+    inv_copy_in<LOGB, T>(op, c, sm, off);
     inv_passes<0, PASSES, LOGB, T, false>(op, c, sm, LOGB + 1);
     inv_pass<LAST, false, false, LOGB, T, 3 * PASSES, false>(op, c, sm, LOGB + 1);
     cl.sync();
@@ -740,7 +1055,17 @@ __device__ __forceinline__ NttLimb make_limb(const Mod &m, uint32_t sb) {
     l.sroot = m.sroot;
     l.sroot_quo = m.sroot_quo;
     l.sb = sb;
+    l.fp = 0;
+    l.fpm = m.fp;
     return l;
+}
+
+// The FP64 form of a limb mod m for an Op whose stores take canonical outputs: inputs below
+// 2^49, or below 3 q after the Op's own Barrett step (any word below 4 q for inverse
+// transforms with `red_in`).
+__device__ __forceinline__ int fp_form(const Mod &m, bool red_in = false) {
+    if (!m.fp) return 0;
+    return FP_ON | (m.value >= FP_PLAIN_Q ? FP_RED : 0) | (red_in ? FP_RED_IN : 0);
 }
 
 constexpr int MAX_LOGB = 14;  // 16384 coefficients = 128 KB of shared memory per CTA
@@ -931,6 +1256,18 @@ inline int small_launch_variant(int v, unsigned blocks) {
     return (v < 3 && small_launch_pairs() && 2 * blocks <= (unsigned)sm_count()) ? v + 3 : v;
 }
 
+// A launch of many limbs of 2^12 or 2^13 coefficients with half the threads per limb, two
+// groups a thread and pass: twice as many limbs share an SM (2^13: 2 of 512 threads, 2^12:
+// 4 of 256), and one limb's loads, barriers and stores overlap another's arithmetic. 256
+// polynomials x 6 limbs at N = 8192: forward 124 -> 95 us, inverse 121 -> 105 us. Below one
+// and a half waves of them the longer limbs cost more than they overlap (66 limbs: 58 ->
+// 62 us, 396 limbs: 33 -> 38 us, 528 limbs: 45 -> 37 us).
+inline int large_launch_variant(int v, int logb, unsigned blocks) {
+    if (v != 0) return v;
+    const unsigned sms = (unsigned)sm_count();
+    return (logb == 13 && blocks >= 3 * sms) || (logb == 12 && blocks >= 6 * sms) ? 1 : 0;
+}
+
 // Dispatch on log2 of the CTA block (1 .. 14); block sizes 2^12 .. 2^14 carry variants
 // with half and a quarter of the threads and their CTA-pair forms. 15, 16, 17: whole
 // limbs of 2^15, 2^16, 2^17 coefficients on CTA pairs and clusters of 4 and 8 CTAs
@@ -942,7 +1279,7 @@ cudaError_t dispatch_ntt(int logb, const Op &op, unsigned blocks, int s0_or_logn
         return launch_ntt<FWD, B, 0>(op, blocks, s0_or_logn, scale_last, s);
 #define TB_CASE2(B)                                                                  \
     case B:                                                                          \
-        switch (small_launch_variant(ntt_variant(FWD, B), blocks)) {                 \
+        switch (large_launch_variant(small_launch_variant(ntt_variant(FWD, B), blocks), B, blocks)) { \
         case 1:                                                                      \
             return launch_ntt<FWD, B, 1>(op, blocks, s0_or_logn, scale_last, s);     \
         case 2:                                                                      \

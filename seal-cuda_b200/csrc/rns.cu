@@ -72,6 +72,7 @@ struct LastInttOp {
     __device__ Ctx ctx(int b) const {
         Ctx c;
         c.lm = make_limb(mods[L - 1], 0);
+        c.lm.fp = fp_form(mods[L - 1]);
         c.in = in + (size_t)(b / size) * istride + ((size_t)((b % size) * L + L - 1) << logn);
         c.out = r + ((size_t)b << logn);
         c.islack = 1;
@@ -101,6 +102,7 @@ struct RescaleNttOp {
     const Mod *mods;
     const DropC *drop;
     int L, K, logn, size;
+    int P;   // polynomials of the launch
     struct Ctx {
         NttLimb lm;
         const uint64_t *in, *r;
@@ -113,14 +115,16 @@ struct RescaleNttOp {
     };
     static constexpr bool wide_slack = true;
     __device__ Ctx ctx(int b) const {
-        const int j = b % (L - 1), p = b / (L - 1);
+        const int j = b / P, p = b % P;   // modulus by modulus
         const Mod &m = mods[j];
         Ctx c;
         c.lm = make_limb(m, 0);
         c.ratio_hi = m.ratio_hi;
         c.d = drop[(size_t)L * K + j];
         c.reduce = mods[L - 1].value > m.value;
-        c.slack = (logn <= MAX_LOGB && m.value < (1ull << 57)) ? SLACK_WIDE : m.value < (1ull << 60) ? SLACK_M : 0;
+        c.lm.fp = fp_form(m);
+        c.slack = c.lm.fp ? 0 : (logn <= MAX_LOGB && m.value < (1ull << 57)) ? SLACK_WIDE
+                              : m.value < (1ull << 60) ? SLACK_M : 0;
         c.wide_off = (m.ratio_hi - 1) * m.value;
         const size_t cb = p / size, k = p % size;
         c.in = in + cb * istride + ((k * L + j) << logn);
@@ -237,7 +241,7 @@ int rescale_to_next(Context &c, int L, const uint64_t *in, uint64_t cstride_in, 
         }
         if (e == cudaSuccess) {
             TraceScope ts("rescale_ntt", s);
-            RescaleNttOp b{in, cstride_in, out, cstride_out, r, c.d_mods, c.d_drop, L, K, c.logn, size};
+            RescaleNttOp b{in, cstride_in, out, cstride_out, r, c.d_mods, c.d_drop, L, K, c.logn, size, (int)P};
             e = dispatch_ntt<true>(c.logn, b, (unsigned)(P * (L - 1)), 0, 0, s);
         }
         cudaFreeAsync(r, s);

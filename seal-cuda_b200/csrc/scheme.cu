@@ -54,6 +54,7 @@ struct InplaceOp {
     __device__ Ctx ctx(int b) const {
         Ctx c;
         c.lm = make_limb(mods[b % L], 0);
+        if (!lazy) c.lm.fp = fp_form(mods[b % L], !FWD);
         c.p = buf + ((size_t)b << logn);
         return c;
     }
