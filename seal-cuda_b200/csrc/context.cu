@@ -22,6 +22,13 @@ int status_from(cudaError_t e) {
     return set_error(TB_ERR_CUDA, cudaGetErrorString(e));
 }
 
+int refuse_capture(cudaStream_t s) {
+    cudaStreamCaptureStatus cap;
+    const cudaError_t e = cudaStreamIsCapturing(s, &cap);
+    if (e != cudaSuccess) return status_from(e);
+    return cap == cudaStreamCaptureStatusNone ? TB_OK : status_from(cudaErrorStreamCaptureUnsupported);
+}
+
 Context::~Context() {
     int prev = 0;
     cudaGetDevice(&prev);
@@ -33,6 +40,7 @@ Context::~Context() {
         if (lv.d_consts) cudaFree(lv.d_consts);
         if (lv.d_bsk_mods) cudaFree(lv.d_bsk_mods);
         if (lv.d_bsk_idx) cudaFree(lv.d_bsk_idx);
+        if (lv.d_compose) cudaFree(lv.d_compose);
     }
     if (d_drop) cudaFree(d_drop);
     if (d_mods) cudaFree(d_mods);

@@ -28,6 +28,8 @@ enum Status {
 
 int status_from(cudaError_t e);
 int set_error(int status, const std::string &msg);
+// The status of a call that does not run inside a stream capture (TB_OK outside one).
+int refuse_capture(cudaStream_t s);
 
 // Offsets (in words) of the per-level RNS constants inside RnsLevel::d_consts.
 // "pair" entries are Shoup operands stored as consecutive {operand, quotient}.
@@ -74,6 +76,7 @@ struct RnsLevel {
     uint64_t *d_consts = nullptr;
     Mod *d_bsk_mods = nullptr;  // Bsk = [B_0 .. B_{bB-1}, m_sk]
     int *d_bsk_idx = nullptr;   // table indices of the Bsk primes
+    uint64_t *d_compose = nullptr;  // CKKS decode: CRT constants of this level (ckks.cu), on first use
     Mod gamma_mod{};            // Barrett ratio only
 };
 
@@ -107,7 +110,7 @@ struct Context {
     // Galois NTT-domain permutation tables, built on first use per element.
     std::mutex galois_mu;
     std::unordered_map<uint32_t, uint32_t *> galois_ntt;
-    uint32_t *d_slot_map = nullptr;   // batch-encoder slot -> coefficient map
+    uint32_t *d_slot_map = nullptr;   // encoder slot -> coefficient map [N] and its inverse [N]
     void *d_fft_roots = nullptr;      // CKKS special-FFT roots: [N] forward, [N] inverse (double2)
     uint64_t *noalloc_scratch = nullptr;  // device address of the static relinearize scratch on `device`
     ~Context();

@@ -103,9 +103,11 @@ struct RescaleNttOp {
     const DropC *drop;
     int L, K, logn, size;
     int P;   // polynomials of the launch
+    const uint64_t *plain;   // encryption: plaintexts ([L-1][N], pstride words apart) added to
+    uint64_t pstride;        // the first polynomial of each ciphertext, or null
     struct Ctx {
         NttLimb lm;
-        const uint64_t *in, *r;
+        const uint64_t *in, *r, *plain;
         uint64_t *out;
         uint64_t ratio_hi;
         DropC d;
@@ -130,6 +132,7 @@ struct RescaleNttOp {
         c.in = in + cb * istride + ((k * L + j) << logn);
         c.out = out + cb * ostride + ((k * (L - 1) + j) << logn);
         c.r = r + ((size_t)p << logn);
+        c.plain = plain && !k ? plain + cb * pstride + ((size_t)j << logn) : nullptr;
         return c;
     }
     // the transform takes any input below 4 q_j: the Barrett remainder (< 2 q_j) plus fix
@@ -156,7 +159,11 @@ struct RescaleNttOp {
         return mul_shoup(x, c.d.inv, c.d.inv_quo, q);
     }
     __device__ void store2(const Ctx &c, int e, uint64_t a, uint64_t b, const Epi &p) const {
-        *reinterpret_cast<ulonglong2 *>(c.out + e) = make_ulonglong2(fin(c, p.in.x, a), fin(c, p.in.y, b));
+        ulonglong2 v = make_ulonglong2(fin(c, p.in.x, a), fin(c, p.in.y, b));
+        if (c.plain) {
+            v = make_ulonglong2(add_mod(v.x, c.plain[e], c.lm.q), add_mod(v.y, c.plain[e + 1], c.lm.q));
+        }
+        *reinterpret_cast<ulonglong2 *>(c.out + e) = v;
     }
 };
 
@@ -215,9 +222,11 @@ __global__ void mod_switch_coeff_kernel(const uint64_t *__restrict__ in, uint64_
 void ensure_pool_retains(int device);
 
 // Drops the last prime of `size` polynomials of B ciphertexts at level L (L limbs in,
-// L-1 limbs out); ciphertext b at in + b*cstride_in, its polynomials L*n apart.
-int rescale_to_next(Context &c, int L, const uint64_t *in, uint64_t cstride_in, uint64_t *out, uint64_t cstride_out,
-                    int size, uint64_t B, cudaStream_t s) {
+// L-1 limbs out); ciphertext b at in + b*cstride_in, its polynomials L*n apart. CKKS:
+// plain, if given, is added to the first polynomial of each result ([L-1][n] per
+// ciphertext, pstride words apart).
+int rescale_add(Context &c, int L, const uint64_t *in, uint64_t cstride_in, uint64_t *out, uint64_t cstride_out,
+                int size, uint64_t B, const uint64_t *plain, uint64_t pstride, cudaStream_t s) {
     const int K = (int)c.chain.size();
     if (L < 2 || L > K) return set_error(TB_ERR_INVALID_ARGUMENT, "nothing to drop at this level");
     if (!in || !out) return set_error(TB_ERR_INVALID_ARGUMENT, "null buffer");
@@ -241,7 +250,8 @@ int rescale_to_next(Context &c, int L, const uint64_t *in, uint64_t cstride_in, 
         }
         if (e == cudaSuccess) {
             TraceScope ts("rescale_ntt", s);
-            RescaleNttOp b{in, cstride_in, out, cstride_out, r, c.d_mods, c.d_drop, L, K, c.logn, size, (int)P};
+            RescaleNttOp b{in, cstride_in, out, cstride_out, r, c.d_mods, c.d_drop, L, K, c.logn, size, (int)P, plain,
+                           pstride};
             e = dispatch_ntt<true>(c.logn, b, (unsigned)(P * (L - 1)), 0, 0, s);
         }
         cudaFreeAsync(r, s);
@@ -254,6 +264,11 @@ int rescale_to_next(Context &c, int L, const uint64_t *in, uint64_t cstride_in, 
                                                                   c.d_drop, c.t_mod, bgv ? c.inv_qlast_t[L] : 0, L,
                                                                   K, c.logn, bgv, P, size);
     return status_from(cudaGetLastError());
+}
+
+int rescale_to_next(Context &c, int L, const uint64_t *in, uint64_t cstride_in, uint64_t *out, uint64_t cstride_out,
+                    int size, uint64_t B, cudaStream_t s) {
+    return rescale_add(c, L, in, cstride_in, out, cstride_out, size, B, nullptr, 0, s);
 }
 
 }  // namespace tb

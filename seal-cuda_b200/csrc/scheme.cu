@@ -20,8 +20,8 @@ namespace tb {
 
 unsigned grid_for(uint64_t work, int threads);
 void ensure_pool_retains(int device);
-int rescale_to_next(Context &c, int L, const uint64_t *in, uint64_t cstride_in, uint64_t *out, uint64_t cstride_out,
-                    int size, uint64_t B, cudaStream_t s);
+int rescale_add(Context &c, int L, const uint64_t *in, uint64_t cstride_in, uint64_t *out, uint64_t cstride_out,
+                int size, uint64_t B, const uint64_t *plain, uint64_t pstride, cudaStream_t s);
 int galois_ntt_table(Context &c, uint32_t elt, const uint32_t **out);
 
 namespace {
@@ -89,6 +89,303 @@ cudaError_t transform(const Context &c, uint64_t *buf, uint64_t polys, int first
     return dispatch_ntt<FWD>(c.logn, op, (unsigned)(polys * L), FWD ? 0 : c.logn, 1, s);
 }
 
+// Transforms fused with what an encryption or a decryption does before and after them.
+// The operations' separate kernels (one or two per ciphertext and step) were bound by
+// their launches: a batch of 16 ciphertexts at N = 16384, L = 8 took 685 us to encrypt, of
+// which the transforms' integer work is about 80.
+
+// Signed small value as a residue.
+__device__ __forceinline__ uint64_t small_residue(int v, uint64_t q) { return v < 0 ? q + (int64_t)v : (uint64_t)v; }
+
+// [0, q) from a transform's output in [0, 4q) (lazy forward, wide inverse) or [0, q)
+__device__ __forceinline__ uint64_t canonical4(uint64_t v, uint64_t q) { return csub(csub(v, 2 * q), q); }
+
+// NTT of the ternary polynomial u of each encryption (small [count][3][N], signed), written
+// as u pk_0 and u pk_1 into t [count][2][L][N].
+struct EncryptUOp {
+    const int32_t *small;
+    const uint64_t *pk;   // [2][K][N]
+    uint64_t *t;
+    const Mod *mods;
+    int L, K, logn;
+    uint32_t count;
+    struct Ctx {
+        NttLimb lm;
+        Mod m;
+        const int32_t *in;
+        const uint64_t *pk0, *pk1;
+        uint64_t *t0, *t1;
+    };
+    __device__ Ctx ctx(int b) const {
+        const uint32_t l = (uint32_t)b / count, cb = (uint32_t)b - l * count;
+        Ctx c;
+        c.m = mods[l];
+        c.lm = make_limb(mods[l], 0);
+        c.lm.fp = fp_form(mods[l]);
+        c.in = small + ((size_t)cb * 3 << logn);
+        c.pk0 = pk + ((size_t)l << logn);
+        c.pk1 = c.pk0 + ((size_t)K << logn);
+        c.t0 = t + (((size_t)cb * 2 * L + l) << logn);
+        c.t1 = c.t0 + ((size_t)L << logn);
+        return c;
+    }
+    __device__ uint64_t load(const Ctx &c, int e) const { return small_residue(c.in[e], c.lm.q); }
+    struct Epi {
+        ulonglong2 a, b;
+    };
+    __device__ Epi epi2(const Ctx &c, int e) const {
+        return {make_ulonglong2(__ldg(c.pk0 + e), __ldg(c.pk0 + e + 1)), make_ulonglong2(__ldg(c.pk1 + e), __ldg(c.pk1 + e + 1))};
+    }
+    __device__ void store2(const Ctx &c, int e, uint64_t x, uint64_t y, const Epi &p) const {
+        *reinterpret_cast<ulonglong2 *>(c.t0 + e) = make_ulonglong2(mul_mod(x, p.a.x, c.m), mul_mod(y, p.a.y, c.m));
+        *reinterpret_cast<ulonglong2 *>(c.t1 + e) = make_ulonglong2(mul_mod(x, p.b.x, c.m), mul_mod(y, p.b.y, c.m));
+    }
+};
+
+// CKKS: t[b][j] += NTT(e_j), the noise polynomials at small [count][1 + j].
+struct EncryptNoiseOp {
+    const int32_t *small;
+    uint64_t *t;
+    const Mod *mods;
+    int L, logn;
+    uint32_t count;
+    struct Ctx {
+        NttLimb lm;
+        const int32_t *in;
+        uint64_t *t;
+    };
+    __device__ Ctx ctx(int b) const {
+        const uint32_t l = (uint32_t)b / (2 * count), p = (uint32_t)b - l * 2 * count, cb = p >> 1, j = p & 1;
+        Ctx c;
+        c.lm = make_limb(mods[l], 0);
+        c.lm.fp = fp_form(mods[l]);
+        c.in = small + (((size_t)cb * 3 + 1 + j) << logn);
+        c.t = t + (((size_t)p * L + l) << logn);
+        return c;
+    }
+    __device__ uint64_t load(const Ctx &c, int e) const { return small_residue(c.in[e], c.lm.q); }
+    struct Epi {
+        ulonglong2 t;
+    };
+    __device__ Epi epi2(const Ctx &c, int e) const { return {*reinterpret_cast<const ulonglong2 *>(c.t + e)}; }
+    __device__ void store2(const Ctx &c, int e, uint64_t x, uint64_t y, const Epi &p) const {
+        const uint64_t q = c.lm.q;
+        *reinterpret_cast<ulonglong2 *>(c.t + e) =
+            make_ulonglong2(add_mod(p.t.x, canonical4(x, q), q), add_mod(p.t.y, canonical4(y, q), q));
+    }
+};
+
+// BFV / BGV: t[b][j] out of the NTT domain, plus e_j (times the plain modulus for BGV).
+struct EncryptInttOp {
+    const int32_t *small;
+    uint64_t *t;
+    const Mod *mods;
+    int L, logn;
+    uint32_t count;
+    uint64_t t_scale;
+    struct Ctx {
+        NttLimb lm;
+        Mod m;
+        const int32_t *in;
+        uint64_t *t;
+        uint64_t ts;
+        int islack;
+    };
+    __device__ Ctx ctx(int b) const {
+        const uint32_t l = (uint32_t)b / (2 * count), p = (uint32_t)b - l * 2 * count, cb = p >> 1, j = p & 1;
+        Ctx c;
+        c.m = mods[l];
+        c.lm = make_limb(mods[l], 0);
+        c.lm.fp = fp_form(mods[l]);
+        c.in = small + (((size_t)cb * 3 + 1 + j) << logn);
+        c.t = t + (((size_t)p * L + l) << logn);
+        c.ts = t_scale ? reduce64(t_scale, c.m) : 0;
+        c.islack = 1;
+        return c;
+    }
+    __device__ void load2(const Ctx &c, int e, uint64_t &a, uint64_t &b) const {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(c.t + e);
+        a = v.x;
+        b = v.y;
+    }
+    __device__ void store(const Ctx &c, int e, uint64_t v) const {
+        const uint64_t q = c.lm.q;
+        uint64_t n = small_residue(c.in[e], q);
+        if (c.ts) n = mul_mod(n, c.ts, c.m);
+        c.t[e] = add_mod(canonical4(v, q), n, q);
+    }
+};
+
+// Forward NTT (lazy) of polynomials 1 .. size - 1 of B ciphertexts into x [B][size-1][L][N].
+struct PhaseNttOp {
+    const uint64_t *ct;
+    uint64_t cstride;
+    uint64_t *x;
+    const Mod *mods;
+    int L, logn, size;
+    struct Ctx {
+        NttLimb lm;
+        const uint64_t *in;
+        uint64_t *out;
+    };
+    __device__ Ctx ctx(int b) const {
+        const int l = b % L, p = b / L;
+        const size_t cb = p / (size - 1), k = p % (size - 1);
+        Ctx c;
+        c.lm = make_limb(mods[l], 0);
+        c.lm.fp = fp_form(mods[l]);
+        c.in = ct + cb * cstride + (((k + 1) * L + l) << logn);
+        c.out = x + ((size_t)b << logn);
+        return c;
+    }
+    __device__ uint64_t load(const Ctx &c, int e) const { return c.in[e]; }
+    __device__ void store2(const Ctx &c, int e, uint64_t a, uint64_t b) const {
+        *reinterpret_cast<ulonglong2 *>(c.out + e) = make_ulonglong2(a, b);
+    }
+};
+
+// s (x_1 + s (x_2 + ...)) by Horner's rule: any words x_k below 4 q.
+__device__ __forceinline__ uint64_t horner(const uint64_t *x, size_t step, int terms, uint64_t s, const Mod &m) {
+    uint64_t acc = x[(terms - 1) * step];
+    for (int k = terms - 2; k >= 0; k--) acc = add_mod(mul_mod(acc, s, m), canonical4(x[k * step], m.value), m.value);
+    return mul_mod(acc, s, m);
+}
+
+// Phase of B ciphertexts in coefficient form: INTT(sum_k x_k s^k) + c_0 into out [B][L][N].
+struct PhaseInttOp {
+    const uint64_t *x, *sk, *ct;
+    uint64_t cstride;
+    uint64_t *out;
+    const Mod *mods;
+    int L, logn, size;
+    struct Ctx {
+        NttLimb lm;
+        Mod m;
+        const uint64_t *x, *sk, *c0;
+        uint64_t *out;
+        int islack;
+    };
+    __device__ Ctx ctx(int b) const {
+        const int l = b % L;
+        const size_t cb = b / L;
+        Ctx c;
+        c.m = mods[l];
+        c.lm = make_limb(mods[l], 0);
+        c.lm.fp = fp_form(mods[l]);
+        c.x = x + ((cb * (size - 1) * L + l) << logn);
+        c.sk = sk + ((size_t)l << logn);
+        c.c0 = ct + cb * cstride + ((size_t)l << logn);
+        c.out = out + ((size_t)b << logn);
+        c.islack = 1;
+        return c;
+    }
+    __device__ void load2(const Ctx &c, int e, uint64_t &a, uint64_t &b) const {
+        const size_t step = (size_t)L << logn;
+        a = horner(c.x + e, step, size - 1, c.sk[e], c.m);
+        b = horner(c.x + e + 1, step, size - 1, c.sk[e + 1], c.m);
+    }
+    __device__ void store(const Ctx &c, int e, uint64_t v) const {
+        const uint64_t q = c.lm.q;
+        c.out[e] = add_mod(canonical4(c.c0[e], q), canonical4(v, q), q);
+    }
+};
+
+// Batch encoder: inverse NTT mod t whose load takes coefficient e from slot inv[e] (zero
+// from `count` on), and the forward NTT whose store puts coefficient e into slot inv[e].
+struct BatchEncodeOp {
+    const uint64_t *slots;
+    uint64_t sstride;
+    uint32_t count;
+    uint64_t *out;
+    const uint32_t *inv;
+    const Mod *mods;   // the plain modulus
+    int logn;
+    struct Ctx {
+        NttLimb lm;
+        const uint64_t *in;
+        uint64_t *out;
+    };
+    __device__ Ctx ctx(int b) const {
+        Ctx c;
+        c.lm = make_limb(mods[0], 0);
+        c.lm.fp = fp_form(mods[0], true);
+        c.in = slots + (size_t)b * sstride;
+        c.out = out + ((size_t)b << logn);
+        return c;
+    }
+    __device__ void load2(const Ctx &c, int e, uint64_t &a, uint64_t &b) const {
+        const uint32_t i = __ldg(inv + e), j = __ldg(inv + e + 1);
+        a = i < count ? c.in[i] : 0;
+        b = j < count ? c.in[j] : 0;
+    }
+    __device__ void store(const Ctx &c, int e, uint64_t v) const { c.out[e] = csub(v, c.lm.q); }
+};
+
+struct BatchDecodeOp {
+    const uint64_t *in;
+    uint64_t *slots;
+    uint64_t sstride;
+    const uint32_t *inv;
+    const Mod *mods;
+    int logn;
+    struct Ctx {
+        NttLimb lm;
+        const uint64_t *in;
+        uint64_t *out;
+    };
+    __device__ Ctx ctx(int b) const {
+        Ctx c;
+        c.lm = make_limb(mods[0], 0);
+        c.lm.fp = fp_form(mods[0]);
+        c.in = in + ((size_t)b << logn);
+        c.out = slots + (size_t)b * sstride;
+        return c;
+    }
+    __device__ uint64_t load(const Ctx &c, int e) const { return c.in[e]; }
+    __device__ void store2(const Ctx &c, int e, uint64_t a, uint64_t b) const {
+        c.out[__ldg(inv + e)] = canonical4(a, c.lm.q);
+        c.out[__ldg(inv + e + 1)] = canonical4(b, c.lm.q);
+    }
+};
+
+// Centred lift of BFV / BGV plaintexts (see plain_lift_kernel) in the load of the NTT.
+struct PlainLiftOp {
+    const uint64_t *plain;
+    uint64_t pstride;
+    uint32_t pcount;
+    uint64_t *out;
+    const Mod *mods;
+    const uint64_t *incr;   // Q - t mod q_l
+    uint64_t thr;           // (t + 1) / 2
+    int L, logn;
+    struct Ctx {
+        NttLimb lm;
+        uint64_t ratio_hi, incr;
+        const uint64_t *in;
+        uint64_t *out;
+    };
+    __device__ Ctx ctx(int b) const {
+        const int l = b % L;
+        Ctx c;
+        c.lm = make_limb(mods[l], 0);
+        c.lm.fp = fp_form(mods[l]);
+        c.ratio_hi = mods[l].ratio_hi;
+        c.incr = incr[l];
+        c.in = plain + (size_t)(b / L) * pstride;
+        c.out = out + ((size_t)b << logn);
+        return c;
+    }
+    __device__ uint64_t load(const Ctx &c, int e) const {
+        if ((uint32_t)e >= pcount) return 0;
+        const uint64_t p = c.in[e], q = c.lm.q;
+        const uint64_t r = csub(p - mulhi(p, c.ratio_hi) * q, q);
+        return p >= thr ? add_mod(r, c.incr, q) : r;
+    }
+    __device__ void store2(const Ctx &c, int e, uint64_t a, uint64_t b) const {
+        *reinterpret_cast<ulonglong2 *>(c.out + e) = make_ulonglong2(canonical4(a, c.lm.q), canonical4(b, c.lm.q));
+    }
+};
+
 // ---------------------------------------------------------------- element-wise
 
 // Index w of a limb-major layout split by units of d limbs of 2^logn words:
@@ -127,6 +424,33 @@ __global__ void dyadic_bcast_kernel(const uint64_t *__restrict__ a, const uint64
     }
 }
 
+// CKKS phase sum_k c_k s^k of B ciphertexts of `size` polynomials into out (ostride words
+// apart) [L][N].
+__global__ void ckks_phase_kernel(const uint64_t *__restrict__ ct, uint64_t cstride, const uint64_t *__restrict__ sk,
+                                  uint64_t *__restrict__ out, uint64_t ostride, const Mod *__restrict__ mods, int L,
+                                  int logn, int size, uint64_t B) {
+    const uint64_t total = (B * L) << logn, pl = (uint64_t)L << logn;
+    for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < total; w += (uint64_t)gridDim.x * blockDim.x) {
+        uint64_t b, r;
+        split_limbs(w, (uint32_t)L, logn, b, r);
+        const Mod &m = mods[r >> logn];
+        const uint64_t *c = ct + b * cstride + r;
+        out[b * ostride + r] = add_mod(*c, horner(c + pl, pl, size - 1, sk[r], m), m.value);
+    }
+}
+
+// Symmetric encryptions: c0 = s c1 for B ciphertexts (c1 at ct + b*cstride + L*N).
+__global__ void sk_product_kernel(uint64_t *__restrict__ ct, uint64_t cstride, const uint64_t *__restrict__ sk,
+                                  const Mod *__restrict__ mods, int L, int logn, uint64_t B) {
+    const uint64_t total = (B * L) << logn, pl = (uint64_t)L << logn;
+    for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < total; w += (uint64_t)gridDim.x * blockDim.x) {
+        uint64_t b, r;
+        split_limbs(w, (uint32_t)L, logn, b, r);
+        uint64_t *c = ct + b * cstride + r;
+        *c = mul_mod(c[pl], sk[r], mods[r >> logn]);
+    }
+}
+
 // op: 0 add, 1 sub, 2 negate (b unused); polynomials of B ciphertexts with strides.
 __global__ void addsub_kernel(const uint64_t *__restrict__ a, uint64_t astride, const uint64_t *__restrict__ b,
                               uint64_t bstride, uint64_t *__restrict__ out, uint64_t ostride,
@@ -144,17 +468,6 @@ __global__ void addsub_kernel(const uint64_t *__restrict__ a, uint64_t astride, 
         else if (op == 1) y = sub_mod(x, b[cb * bstride + r], q);
         else y = neg_mod(x, q);
         out[cb * ostride + r] = y;
-    }
-}
-
-// x += e (BFV/CKKS) or x += t*e mod q (BGV), over P packed polynomials.
-__global__ void add_noise_kernel(uint64_t *__restrict__ x, const uint64_t *__restrict__ e, const Mod *__restrict__ mods,
-                                 int L, int logn, uint64_t total, uint64_t t_scale) {
-    for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < total; w += (uint64_t)gridDim.x * blockDim.x) {
-        const Mod m = mods[limb_of(w, logn, L)];
-        uint64_t v = e[w];
-        if (t_scale) v = mul_mod(v, reduce64(t_scale, m), m);
-        x[w] = add_mod(x[w], v, m.value);
     }
 }
 
@@ -293,28 +606,6 @@ __global__ void plain_lift_kernel(const uint64_t *__restrict__ plain, uint64_t p
     }
 }
 
-// Slot <-> coefficient permutation of the batch encoder (src/batchencoder.cpp:64-82).
-__global__ void slot_scatter_kernel(const uint64_t *__restrict__ slots, uint64_t sstride, uint32_t count,
-                                    uint64_t *__restrict__ out, const uint32_t *__restrict__ map, uint32_t n,
-                                    uint64_t t, uint64_t B) {
-    const uint64_t total = B * n;
-    for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < total; w += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t b = w / n;
-        const uint32_t i = (uint32_t)(w - b * n);
-        out[b * n + map[i]] = i < count ? slots[b * sstride + i] : 0;
-    }
-}
-
-__global__ void slot_gather_kernel(const uint64_t *__restrict__ coeffs, uint64_t *__restrict__ slots, uint64_t sstride,
-                                   const uint32_t *__restrict__ map, uint32_t n, uint64_t B) {
-    const uint64_t total = B * n;
-    for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < total; w += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t b = w / n;
-        const uint32_t i = (uint32_t)(w - b * n);
-        slots[b * sstride + i] = coeffs[b * n + map[i]];
-    }
-}
-
 __global__ void galois_ntt_poly_kernel(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
                                        const uint32_t *__restrict__ perm, int logn, uint64_t P) {
     const uint64_t total = P << logn;
@@ -354,8 +645,14 @@ int slot_map(Context &c, const uint32_t **out) {
             map[n / 2 + i] = host::bitrev((uint32_t)((m - pos - 1) >> 1), c.logn);
             pos = (pos * 3) & (m - 1);
         }
-        cudaError_t e = cudaMalloc(&c.d_slot_map, n * 4);
-        if (e == cudaSuccess) e = cudaMemcpy(c.d_slot_map, map.data(), n * 4, cudaMemcpyHostToDevice);
+        // the map (slot -> coefficient) and its inverse
+        map.resize(2 * n);
+        for (uint32_t i = 0; i < n; i++) map[n + map[i]] = i;
+        uint32_t *d = nullptr;
+        cudaError_t e = cudaMalloc(&d, 2ull * n * 4);
+        if (e == cudaSuccess) e = cudaMemcpy(d, map.data(), 2ull * n * 4, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) c.d_slot_map = d;
+        else if (d) cudaFree(d);
         if (e != cudaSuccess) return status_from(e);
     }
     *out = c.d_slot_map;
@@ -405,16 +702,13 @@ int encrypt_zero_symmetric(Context &c, const uint64_t *seed8, const uint64_t *sk
     // public seed = first 64 bytes of the bootstrap stream; c1 = uniform from it
     e = cudaMemsetAsync(ps, 0, sizeof(PrngState) * count, s);
     if (e != cudaSuccess) return status_from(e);
-    for (int b = 0; b < count; b++) {
-        r = prng_bytes(bs + b, 64, reinterpret_cast<uint8_t *>(ps + b), s);   // seed is the first member
-        if (r != TB_OK) return r;
-    }
+    // the seed is the state's first member
+    r = prng_bytes(bs, count, 64, reinterpret_cast<uint8_t *>(ps), sizeof(PrngState), s);
+    if (r != TB_OK) return r;
     if (seeds) {
         uint8_t *words = sw.as<uint8_t>();
-        for (int b = 0; b < count; b++) {
-            r = prng_bytes(ps + b, 16, words + 16 * b, s);
-            if (r != TB_OK) return r;
-        }
+        r = prng_bytes(ps, count, 16, words, 16, s);
+        if (r != TB_OK) return r;
         std::vector<uint32_t> host(4ull * count);
         e = cudaMemcpyAsync(host.data(), words, 16ull * count, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -431,34 +725,27 @@ int encrypt_zero_symmetric(Context &c, const uint64_t *seed8, const uint64_t *sk
         e = cudaGetLastError();
         if (e != cudaSuccess) return status_from(e);
     } else {
-        for (int b = 0; b < count; b++) {
-            r = sample_poly(c, SAMPLE_UNIFORM, ps + b, 1, 0, L, out + b * ostride + (uint64_t)L * n, 0, s);
-            if (r != TB_OK) return r;
-        }
+        r = sample_poly(c, SAMPLE_UNIFORM, ps, count, 0, L, out + (uint64_t)L * n, ostride, s);
+        if (r != TB_OK) return r;
     }
     r = sample_poly(c, SAMPLE_CBD, bs, count, 0, L, noise.as<uint64_t>(), 0, s);
     if (r != TB_OK) return r;
     // c0 = sk * c1 (NTT domain)
-    for (int b = 0; b < count; b++) {
-        dyadic_bcast_kernel<<<grid_for((uint64_t)L * n, 256), 256, 0, s>>>(out + b * ostride + (uint64_t)L * n, sk,
-                                                                         out + b * ostride, c.d_mods, L, c.logn, 1,
-                                                                         1, 0);
-    }
-    if (ntt) {
-        e = transform<true>(c, noise.as<uint64_t>(), count, 0, L, false, s);
-    } else {
-        for (int b = 0; b < count && e == cudaSuccess; b++) e = transform<false>(c, out + b * ostride, 1, 0, L, false, s);
+    sk_product_kernel<<<grid_for((uint64_t)count * L * n, 256), 256, 0, s>>>(out, ostride, sk, c.d_mods, L, c.logn,
+                                                                           count);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) {
+        if (ntt) e = transform<true>(c, noise.as<uint64_t>(), count, 0, L, false, s);
+        else if (ostride == 2ull * L * n) e = transform<false>(c, out, 2ull * count, 0, L, false, s);   // c0 and c1
+        else
+            for (int b = 0; b < count && e == cudaSuccess; b++) e = transform<false>(c, out + b * ostride, 2, 0, L, false, s);
     }
     if (e != cudaSuccess) return status_from(e);
     const uint64_t tsc = c.scheme == SCHEME_BGV ? c.t : 0;
     neg_sum_kernel<<<grid_for((uint64_t)count * L * n, 256), 256, 0, s>>>(out, noise.as<uint64_t>(), c.d_mods, L,
                                                                          c.logn, (uint64_t)count * L * n, tsc,
                                                                          ostride, (uint64_t)L * n);
-    if (!ntt)
-        for (int b = 0; b < count && e == cudaSuccess; b++)
-            e = transform<false>(c, out + b * ostride + (uint64_t)L * n, 1, 0, L, false, s);
-    if (e == cudaSuccess) e = cudaGetLastError();
-    return status_from(e);
+    return status_from(cudaGetLastError());
 }
 
 int keygen_public(Context &c, const uint64_t *seed8, const uint64_t *sk, uint64_t *pk, cudaStream_t s) {
@@ -516,54 +803,45 @@ int encrypt(Context &c, const uint64_t *seed8, const uint64_t *pk, int L, const 
     if (!ostride) ostride = 2ull * L * n;
     const bool ckks = c.scheme == SCHEME_CKKS;
     const int Lp = L < K ? L + 1 : L;   // encrypt one level up, then drop its last prime
+    if (count * 2 * Lp > 0x7fffffffull) return set_error(TB_ERR_INVALID_ARGUMENT, "too many ciphertexts in one call");
+    const RnsLevel &lv = c.levels[L];
+    const int mode = c.scheme == SCHEME_BFV ? 0 : (c.scheme == SCHEME_BGV ? 1 : 2);
     ensure_pool_retains(c.device);
-    DevBuf st(s), u(s), tmp(s), en(s);
+    DevBuf st(s), small(s), tmp(s);
     cudaError_t e = st.alloc(sizeof(PrngState) * count);
-    if (e == cudaSuccess) e = u.alloc(8ull * count * Lp * n);
+    if (e == cudaSuccess) e = small.alloc(3ull * sizeof(int32_t) * count * n);
     if (e == cudaSuccess) e = tmp.alloc(8ull * count * 2 * Lp * n);
-    if (e == cudaSuccess) e = en.alloc(8ull * count * Lp * n);
     if (e != cudaSuccess) return status_from(e);
     PrngState *ps = st.as<PrngState>();
+    int32_t *sm = small.as<int32_t>();
+    uint64_t *T = tmp.as<uint64_t>();
     int r = prng_init(ps, (int)count, seed8, s);
     if (r != TB_OK) return r;
     TraceScope ts("encrypt", s);
-    uint64_t *U = u.as<uint64_t>(), *T = tmp.as<uint64_t>(), *E = en.as<uint64_t>();
-    r = sample_poly(c, SAMPLE_TERNARY, ps, (int)count, 0, Lp, U, 0, s);
+    r = sample_encryption(c, ps, (int)count, sm, s);
     if (r != TB_OK) return r;
-    e = transform<true>(c, U, count, 0, Lp, false, s);
+    // T[b][j] = u * pk_j (pk limbs 0..Lp-1 of the key-level public key) + e_j
+    EncryptUOp ou{sm, pk, T, c.d_mods, Lp, K, c.logn, (uint32_t)count};
+    e = dispatch_ntt<true>(c.logn, ou, (unsigned)(count * Lp), 0, 0, s);
     if (e != cudaSuccess) return status_from(e);
-    // T[b][j] = u * pk_j (pk limbs 0..Lp-1 of the key-level public key)
-    for (int j = 0; j < 2; j++) {
-        for (uint64_t b = 0; b < count; b++) {
-            dyadic_bcast_kernel<<<grid_for((uint64_t)Lp * n, 256), 256, 0, s>>>(
-                U + b * Lp * n, pk + (uint64_t)j * K * n, T + (b * 2 + j) * Lp * n, c.d_mods, Lp, c.logn, 1, 1, 0);
-        }
+    if (ckks) {
+        EncryptNoiseOp on{sm, T, c.d_mods, Lp, c.logn, (uint32_t)count};
+        e = dispatch_ntt<true>(c.logn, on, (unsigned)(count * 2 * Lp), 0, 0, s);
+    } else {
+        EncryptInttOp oi{sm, T, c.d_mods, Lp, c.logn, (uint32_t)count, c.scheme == SCHEME_BGV ? c.t : 0};
+        e = dispatch_ntt<false>(c.logn, oi, (unsigned)(count * 2 * Lp), c.logn, 1, s);
     }
-    if (!ckks) {
-        e = transform<false>(c, T, count * 2, 0, Lp, false, s);
-        if (e != cudaSuccess) return status_from(e);
-    }
-    for (int j = 0; j < 2; j++) {
-        r = sample_poly(c, SAMPLE_CBD, ps, (int)count, 0, Lp, E, 0, s);
-        if (r != TB_OK) return r;
-        if (ckks) e = transform<true>(c, E, count, 0, Lp, false, s);
-        if (e != cudaSuccess) return status_from(e);
-        const uint64_t tsc = c.scheme == SCHEME_BGV ? c.t : 0;
-        for (uint64_t b = 0; b < count; b++)
-            add_noise_kernel<<<grid_for((uint64_t)Lp * n, 256), 256, 0, s>>>(T + (b * 2 + j) * Lp * n, E + b * Lp * n,
-                                                                           c.d_mods, Lp, c.logn, (uint64_t)Lp * n, tsc);
-    }
+    if (e != cudaSuccess) return status_from(e);
     if (Lp != L) {
-        r = rescale_to_next(c, Lp, T, 2ull * Lp * n, out, ostride, 2, count, s);
+        r = rescale_add(c, Lp, T, 2ull * Lp * n, out, ostride, 2, count, ckks ? plain : nullptr, pstride, s);
         if (r != TB_OK) return r;
+        if (ckks) return TB_OK;
     } else {
         e = cudaMemcpy2DAsync(out, ostride * 8, T, 2ull * Lp * n * 8, 2ull * Lp * n * 8, count,
                               cudaMemcpyDeviceToDevice, s);
         if (e != cudaSuccess) return status_from(e);
     }
     if (plain) {
-        const RnsLevel &lv = c.levels[L];
-        const int mode = c.scheme == SCHEME_BFV ? 0 : (c.scheme == SCHEME_BGV ? 1 : 2);
         if (mode == 0 && !lv.d_consts) return set_error(TB_ERR_UNSUPPORTED, "plain modulus not coprime to q");
         add_plain_kernel<<<grid_for(count * L * n, 256), 256, 0, s>>>(out, ostride, plain, pstride, pcount, c.d_mods,
                                                                       lv.d_consts, lv.off, L, c.logn, c.t, mode, 0,
@@ -657,47 +935,20 @@ int expand_seeded(Context &c, int L, uint64_t seed, bool inverse_ntt, uint64_t *
 
 // ------------------------------------------------------------------ decryption
 
-// phase = sum_k c_k s^k (NTT domain for CKKS; coefficient form for BFV/BGV)
-// (Decryptor::dotProductCtSkArray). out [B][L][N].
+// phase = sum_k c_k s^k in coefficient form (BFV/BGV) (Decryptor::dotProductCtSkArray);
+// c_0 stays out of the transforms. out [B][L][N].
 static int phase(Context &c, const uint64_t *sk, int L, int size, const uint64_t *ct, uint64_t cstride, uint64_t *out,
                  uint64_t B, cudaStream_t s) {
-    const uint64_t n = c.n;
-    const bool ckks = c.scheme == SCHEME_CKKS;
-    const uint64_t pl = (uint64_t)L * n;
-    DevBuf pw(s), tmp(s);
-    cudaError_t e = pw.alloc(8ull * pl * 2);   // s^k and scratch
-    if (e == cudaSuccess) e = tmp.alloc(8ull * B * size * pl);
+    if (B * (uint64_t)(size - 1) * L > 0x7fffffffull)
+        return set_error(TB_ERR_INVALID_ARGUMENT, "too many limbs in one launch");
+    DevBuf x(s);
+    cudaError_t e = x.alloc(8ull * B * (size - 1) * L * c.n);
     if (e != cudaSuccess) return status_from(e);
-    uint64_t *T = tmp.as<uint64_t>();
-    e = cudaMemcpy2DAsync(T, size * pl * 8, ct, cstride * 8, size * pl * 8, B, cudaMemcpyDeviceToDevice, s);
+    PhaseNttOp f{ct, cstride, x.as<uint64_t>(), c.d_mods, L, c.logn, size};
+    e = dispatch_ntt<true>(c.logn, f, (unsigned)(B * (size - 1) * L), 0, 0, s);
     if (e != cudaSuccess) return status_from(e);
-    if (!ckks) {
-        e = transform<true>(c, T, B * size, 0, L, false, s);
-        if (e != cudaSuccess) return status_from(e);
-    }
-    // acc = c0; acc += c_k * s^k
-    uint64_t *S = pw.as<uint64_t>(), *S2 = S + pl;
-    e = cudaMemcpy2DAsync(S, pl * 8, sk, pl * 8, pl * 8, 1, cudaMemcpyDeviceToDevice, s);   // s (first L limbs)
-    if (e != cudaSuccess) return status_from(e);
-    e = cudaMemcpy2DAsync(out, pl * 8, T, size * pl * 8, pl * 8, B, cudaMemcpyDeviceToDevice, s);
-    if (e != cudaSuccess) return status_from(e);
-    for (int k = 1; k < size; k++) {
-        for (uint64_t b = 0; b < B; b++) {
-            uint64_t *ck = T + (b * size + k) * pl;
-            dyadic_bcast_kernel<<<grid_for(pl, 256), 256, 0, s>>>(ck, S, ck, c.d_mods, L, c.logn, 1, 1, 0);
-            addsub_kernel<<<grid_for(pl, 256), 256, 0, s>>>(out + b * pl, 0, ck, 0, out + b * pl, 0, c.d_mods, L,
-                                                            c.logn, 1, 1, 0);
-        }
-        if (k + 1 < size) {
-            dyadic_bcast_kernel<<<grid_for(pl, 256), 256, 0, s>>>(S, sk, S2, c.d_mods, L, c.logn, 1, 1, 0);
-            std::swap(S, S2);
-        }
-    }
-    if (!ckks) {
-        e = transform<false>(c, out, B, 0, L, false, s);
-        if (e != cudaSuccess) return status_from(e);
-    }
-    return status_from(cudaGetLastError());
+    PhaseInttOp i{x.as<uint64_t>(), sk, ct, cstride, out, c.d_mods, L, c.logn, size};
+    return status_from(dispatch_ntt<false>(c.logn, i, (unsigned)(B * L), c.logn, 1, s));
 }
 
 // BFV/BGV: plaintext words mod t [B][N] (ostride words apart); CKKS: [B][L][N] NTT form.
@@ -712,13 +963,18 @@ int decrypt(Context &c, const uint64_t *sk, int L, int size, const uint64_t *ct,
     ensure_pool_retains(c.device);
     TraceScope ts("decrypt", s);
     if (c.scheme == SCHEME_CKKS) {
-        if (!ostride || ostride == (uint64_t)L * n) return phase(c, sk, L, size, ct, cstride, out, B, s);
+        if (!ostride) ostride = (uint64_t)L * n;
+        // a result that overlaps the ciphertexts goes through scratch
+        const bool overlap = out < ct + B * cstride && ct < out + B * ostride;
         DevBuf ph(s);
-        cudaError_t e = ph.alloc(8ull * B * L * n);
+        cudaError_t e = overlap ? ph.alloc(8ull * B * L * n) : cudaSuccess;
         if (e != cudaSuccess) return status_from(e);
-        int r = phase(c, sk, L, size, ct, cstride, ph.as<uint64_t>(), B, s);
-        if (r != TB_OK) return r;
-        return status_from(cudaMemcpy2DAsync(out, ostride * 8, ph.p, L * n * 8, L * n * 8, B, cudaMemcpyDeviceToDevice, s));
+        ckks_phase_kernel<<<grid_for(B * L * n, 256), 256, 0, s>>>(ct, cstride, sk, overlap ? ph.as<uint64_t>() : out,
+                                                                       overlap ? (uint64_t)L * n : ostride, c.d_mods, L,
+                                                                       c.logn, size, B);
+        if (overlap)
+            e = cudaMemcpy2DAsync(out, ostride * 8, ph.p, L * n * 8, L * n * 8, B, cudaMemcpyDeviceToDevice, s);
+        return status_from(e == cudaSuccess ? cudaGetLastError() : e);
     }
     if (!ostride) ostride = n;
     const RnsLevel &lv = c.levels[L];
@@ -757,9 +1013,10 @@ int batch_encode(Context &c, const uint64_t *slots, uint64_t sstride, uint32_t c
     const uint32_t *map = nullptr;
     int r = slot_map(c, &map);
     if (r != TB_OK) return r;
+    if (B > 0x7fffffffull) return set_error(TB_ERR_INVALID_ARGUMENT, "too many plaintexts in one call");
     TraceScope ts("batch_encode", s);
-    slot_scatter_kernel<<<grid_for(B * c.n, 256), 256, 0, s>>>(slots, sstride, count, out, map, c.n, c.t, B);
-    return status_from(transform<false>(c, out, B, c.plain_index, 1, false, s));
+    BatchEncodeOp op{slots, sstride, count, out, map + c.n, c.d_mods + c.plain_index, c.logn};
+    return status_from(dispatch_ntt<false>(c.logn, op, (unsigned)B, c.logn, 1, s));
 }
 
 // plaintexts [B][N] -> slots [B][N] (BatchEncoder::decode).
@@ -771,14 +1028,10 @@ int batch_decode(Context &c, const uint64_t *plain, uint64_t *slots, uint64_t ss
     const uint32_t *map = nullptr;
     int r = slot_map(c, &map);
     if (r != TB_OK) return r;
-    DevBuf tmp(s);
-    cudaError_t e = tmp.alloc(8ull * B * c.n);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(tmp.p, plain, 8ull * B * c.n, cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess) e = transform<true>(c, tmp.as<uint64_t>(), B, c.plain_index, 1, false, s);
-    if (e != cudaSuccess) return status_from(e);
+    if (B > 0x7fffffffull) return set_error(TB_ERR_INVALID_ARGUMENT, "too many plaintexts in one call");
     TraceScope ts("batch_decode", s);
-    slot_gather_kernel<<<grid_for(B * c.n, 256), 256, 0, s>>>(tmp.as<uint64_t>(), slots, sstride, map, c.n, B);
-    return status_from(cudaGetLastError());
+    BatchDecodeOp op{plain, slots, sstride, map + c.n, c.d_mods + c.plain_index, c.logn};
+    return status_from(dispatch_ntt<true>(c.logn, op, (unsigned)B, 0, 0, s));
 }
 
 // ------------------------------------------------------------------ plain multiply
@@ -946,11 +1199,10 @@ int plain_to_ntt(Context &c, int L, const uint64_t *plain, uint64_t pstride, uin
     if (!pstride) pstride = pcount;
     const RnsLevel &lv = c.levels[L];
     if (!lv.d_consts) return set_error(TB_ERR_UNSUPPORTED, "plain modulus not coprime to q");
-    const uint64_t pl = (uint64_t)L * c.n;
+    if (B * (uint64_t)L > 0x7fffffffull) return set_error(TB_ERR_INVALID_ARGUMENT, "too many limbs in one launch");
     TraceScope ts("plain_to_ntt", s);
-    plain_lift_kernel<<<grid_for(B * pl, 256), 256, 0, s>>>(plain, pstride, pcount, out, c.d_mods, lv.d_consts,
-                                                            lv.off, c.t, L, c.logn, B);
-    return status_from(transform<true>(c, out, B, 0, L, false, s));
+    PlainLiftOp op{plain, pstride, pcount, out, c.d_mods, lv.d_consts + lv.off.plain_incr, (c.t + 1) >> 1, L, c.logn};
+    return status_from(dispatch_ntt<true>(c.logn, op, (unsigned)(B * L), 0, 0, s));
 }
 
 // Every coefficient of limb l of each of B plaintexts [L][N] set to vals[l].
