@@ -393,6 +393,8 @@ struct ModDownBase {
         int reduce;
         int slack;   // forward transform (CKKS) with deferred reductions
         uint64_t wide_off;   // (floor(2^64 / q_j) - 1) q_j: the epilogue's offset after the wide form
+        int islack;   // inverse transforms (BFV, BGV): the wide form, outputs below 4 q_j: the
+                      // epilogue's Shoup product takes v + 2 q_j - t, below 6 q_j < 2^64
     };
     static constexpr bool wide_slack = true;
     __device__ Ctx make(int b) const {
@@ -408,6 +410,7 @@ struct ModDownBase {
         c.slack = c.lm.fp ? 0 : (logn <= MAX_LOGB && m.value < (1ull << 57)) ? SLACK_WIDE
                               : m.value < (1ull << 60) ? SLACK_M : 0;
         c.wide_off = (m.ratio_hi - 1) * m.value;
+        c.islack = 1;
         c.acc = acc + (((size_t)bc * (L + 1) + j) << logn);
         c.last = last + ((size_t)bc << logn);
         c.ct = ct + (size_t)cb * cstride + (((size_t)cc * L + j) << logn);

@@ -342,22 +342,39 @@ cudaError_t behz_dispatch(int L, uint64_t threads, cudaStream_t s, A... args) {
 }
 #undef TB_BEHZ_CASE
 
-// NTT over a packed [P][limbs][N] buffer; limb l uses mods[l] (chain or Bsk array).
+// A lazy forward transform whose outputs go into the tensor product: its products of two
+// such words, two of them summed, stay below 2^128 and are reduced by the general Barrett
+// step. For q < 2^57 the no-subtraction form qualifies (canonical inputs below q, outputs
+// below 57 q < 2^62.9); for q < 2^60 the outputs below 16 q are brought below 4 q.
+__device__ __forceinline__ int tensor_slack(uint64_t q, int logn) {
+    return (logn <= MAX_LOGB && q < (1ull << 57)) ? SLACK_WIDE : q < (1ull << 60) ? SLACK_M : 0;
+}
+__device__ __forceinline__ uint64_t tensor_word(uint64_t v, uint64_t q, int slack) {
+    return slack == SLACK_M ? csub(csub(v, 8 * q), 4 * q) : v;
+}
+
+// NTT over a packed [P][limbs][N] buffer; limb l uses mods[l] (chain or Bsk array). The
+// inverse transform's words go into the floor kernel's Shoup products, which take any
+// 64-bit word: the wide inverse form, unreduced.
 template <bool FWD>
 struct PackedNttOp {
     const uint64_t *in;
     uint64_t *out;
     const Mod *mods;
     int limbs, logn;
+    static constexpr bool wide_slack = true;
     struct Ctx {
         NttLimb lm;
         const uint64_t *in;
         uint64_t *out;
+        int slack, islack;
     };
     __device__ Ctx ctx(int b) const {
         Ctx c;
         c.lm = make_limb(mods[b % limbs], 0);
         c.lm.fp = fp_form(mods[b % limbs]);
+        c.slack = FWD && !c.lm.fp ? tensor_slack(c.lm.q, logn) : 0;
+        c.islack = !FWD;
         c.in = in + ((size_t)b << logn);
         c.out = out + ((size_t)b << logn);
         return c;
@@ -370,7 +387,8 @@ struct PackedNttOp {
     }
     __device__ void store(const Ctx &c, int e, uint64_t v) const { c.out[e] = v; }
     __device__ void store2(const Ctx &c, int e, uint64_t a, uint64_t b) const {
-        *reinterpret_cast<ulonglong2 *>(c.out + e) = make_ulonglong2(a, b);
+        *reinterpret_cast<ulonglong2 *>(c.out + e) =
+            make_ulonglong2(tensor_word(a, c.lm.q, c.slack), tensor_word(b, c.lm.q, c.slack));
     }
 };
 
@@ -382,10 +400,12 @@ struct PairNttOp {
     uint64_t *out;
     const Mod *mods;
     int L, logn;
+    static constexpr bool wide_slack = true;
     struct Ctx {
         NttLimb lm;
         const uint64_t *in;
         uint64_t *out;
+        int slack;
     };
     __device__ Ctx ctx(int blk) const {
         const int l = blk % L;
@@ -394,6 +414,7 @@ struct PairNttOp {
         Ctx c;
         c.lm = make_limb(mods[l], 0);
         c.lm.fp = fp_form(mods[l]);
+        c.slack = c.lm.fp ? 0 : tensor_slack(c.lm.q, logn);
         c.in = (slot < 2 ? a + (size_t)ct * astride + (((size_t)slot * L + l) << logn)
                          : b + (size_t)ct * bstride + (((size_t)(slot - 2) * L + l) << logn));
         c.out = out + ((size_t)blk << logn);
@@ -401,7 +422,8 @@ struct PairNttOp {
     }
     __device__ uint64_t load(const Ctx &c, int e) const { return c.in[e]; }
     __device__ void store2(const Ctx &c, int e, uint64_t x, uint64_t y) const {
-        *reinterpret_cast<ulonglong2 *>(c.out + e) = make_ulonglong2(x, y);
+        *reinterpret_cast<ulonglong2 *>(c.out + e) =
+            make_ulonglong2(tensor_word(x, c.lm.q, c.slack), tensor_word(y, c.lm.q, c.slack));
     }
 };
 
@@ -417,6 +439,7 @@ struct CtInttOutOp {
         NttLimb lm;
         const uint64_t *in;
         uint64_t *out;
+        int islack;   // the wide inverse form: outputs below 4q
     };
     __device__ Ctx ctx(int b) const {
         const int l = b % L;
@@ -424,6 +447,7 @@ struct CtInttOutOp {
         Ctx c;
         c.lm = make_limb(mods[l], 0);
         c.lm.fp = fp_form(mods[l]);
+        c.islack = 1;
         c.in = in + ((size_t)b << logn);
         c.out = out + (size_t)(p / per) * ostride + (((size_t)(p % per) * L + l) << logn);
         return c;
@@ -433,7 +457,7 @@ struct CtInttOutOp {
         a = v.x;
         b = v.y;
     }
-    __device__ void store(const Ctx &c, int e, uint64_t v) const { c.out[e] = csub(v, c.lm.q); }
+    __device__ void store(const Ctx &c, int e, uint64_t v) const { c.out[e] = csub(csub(v, 2 * c.lm.q), c.lm.q); }
 };
 
 }  // namespace
