@@ -75,27 +75,35 @@ __device__ __forceinline__ double fp_centred(uint64_t w, uint64_t q) {
 // 6, in stage order) of every group side by side, so a warp's loads of one k are
 // consecutive. Radix-8 passes end at the last stage, so the stages before the first one
 // (logn mod 3) keep their natural order. index 1 .. n - 1.
-__host__ __device__ inline uint32_t fp_fwd_index(uint32_t i, int logn) {
-    int s = 0;
-    while ((2u << s) <= i) s++;
+// Natural index i of stage s (2^s <= i < 2^(s+1)).
+__host__ __device__ constexpr uint32_t fp_fwd_stage_index(uint32_t i, int s, int logn) {
     const int r = logn % 3;
     if (s < r) return i;
     const int s0 = r + (s - r) / 3 * 3, t = s - s0;
-    const uint32_t X = i >> t, k = (1u << t) - 1 + (i & ((1u << t) - 1));
-    return (k << s0) + X;
+    return (((1u << t) - 1 + (i & ((1u << t) - 1))) << s0) + (i >> t);
+}
+__host__ __device__ inline uint32_t fp_fwd_index(uint32_t i, int logn) {
+    int s = 0;
+    while ((2u << s) <= i) s++;
+    return fp_fwd_stage_index(i, s, logn);
 }
 
 // Inverse tables: stage sg uses indices n + 1 - (n >> sg) onwards, the radix-8 passes start
-// at stages 0, 3, 6, ... and the remaining last stages keep their natural order.
+// at stages 0, 3, 6, ... and the remaining last stages keep their natural order. b: the
+// twiddle's number in its stage.
+__host__ __device__ constexpr uint32_t fp_inv_stage_index(uint32_t b, int sg, int logn) {
+    const uint32_t n = 1u << logn;
+    const int s = sg / 3 * 3, t = sg - s;
+    if (s + 3 > logn) return n + 1 - (n >> sg) + b;
+    const uint32_t j = b & ((4u >> t) - 1), blk = b >> (2 - t);
+    const uint32_t k = t == 0 ? j : t == 1 ? 4 + j : 6;
+    return n + 1 - (n >> s) + k * (n >> (s + 3)) + blk;
+}
 __host__ __device__ inline uint32_t fp_inv_index(uint32_t i, int logn) {
     const uint32_t n = 1u << logn;
     int sg = 0;
     while (sg + 1 < logn && n + 1 - (n >> (sg + 1)) <= i) sg++;
-    const int s = sg / 3 * 3, t = sg - s;
-    if (s + 3 > logn) return i;
-    const uint32_t b = i - (n + 1 - (n >> sg)), j = b & ((4u >> t) - 1), blk = b >> (2 - t);
-    const uint32_t k = t == 0 ? j : t == 1 ? 4 + j : 6;
-    return n + 1 - (n >> s) + k * (n >> (s + 3)) + blk;
+    return fp_inv_stage_index(i - (n + 1 - (n >> sg)), sg, logn);
 }
 
 }  // namespace tb

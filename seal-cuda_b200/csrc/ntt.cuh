@@ -347,8 +347,7 @@ __device__ __forceinline__ void fwd_group_fp(double (&v)[1 << R_LOG], const Tw &
     }
 }
 
-// Pass of R_LOG stages starting at local stage s (compare fwd_pass). The remainder pass's
-// twiddles are in natural order.
+// Pass of R_LOG stages starting at local stage s (compare fwd_pass).
 // S0: the global stage of local stage 0.
 template <int R_LOG, bool FROM_GLOBAL, int LOGB, int T, int s, int S0, class Op, class Ctx>
 __device__ __forceinline__ void fwd_pass_fp(const Op &op, const Ctx &c, double *sm, const FpPass &f) {
@@ -381,7 +380,7 @@ __device__ __forceinline__ void fwd_pass_fp(const Op &op, const Ctx &c, double *
             [&](int t, int k) {
                 if constexpr (OWN) return make_double2(w[k], __dmul_rn(w[k], f.qinv));
                 else if constexpr (R_LOG == 3) return __ldg(prow + (k << gs));
-                else return __ldg(f.p + ((X << t) + (uint32_t)(k - ((1 << t) - 1))));
+                else return __ldg(f.p + fp_fwd_stage_index((X << t) + (uint32_t)(k - ((1 << t) - 1)), gs + t, S0 + LOGB));
             },
             f);
 #pragma unroll
@@ -652,12 +651,7 @@ __device__ __forceinline__ void inv_pass_fp(const Op &op, const Ctx &c, double *
         const int base = ((g >> s) << (s + R_LOG)) + (g & ((1 << s) - 1));
         const int sb = swz(base);
         const uint32_t blk = (c.lm.sb << (LOGB - s - R_LOG)) + (uint32_t)(g >> s);
-        // radix 8: twiddle k (4, 2, 1 of the three stages); else stages in natural order
-        auto at = [&](int t, int k) -> uint32_t {
-            if constexpr (R_LOG == 3) return n + 1 - (n >> s) + (uint32_t)k * (n >> (s + 3)) + blk;
-            else if constexpr (R_LOG == 2) return t == 0 ? n + 1 - (n >> s) + 2 * blk + (uint32_t)k : n + 1 - (n >> (s + 1)) + blk;
-            else return n + 1 - (n >> s) + blk;
-        };
+        // radix 8: twiddle k (4, 2, 1 of the three stages) of the group
         double w[R];
         if constexpr (OWN) {
 #pragma unroll
@@ -686,7 +680,11 @@ __device__ __forceinline__ void inv_pass_fp(const Op &op, const Ctx &c, double *
                     v[k + h] = fp_mulmod(__dadd_rn(x, -y), sr, __dmul_rn(sr, qinv), q);
                 } else {
                     const int ki = R - (R >> t) + (k >> (t + 1));
-                    const double2 m = OWN ? make_double2(w[ki], __dmul_rn(w[ki], qinv)) : (R_LOG == 3 ? __ldg(f.p + blk + (n + 1 - (n >> s) - skip + (uint32_t)ki * (n >> (s + 3)))) : __ldg(f.p + (at(t, ki) - skip)));
+                    const double2 m =
+                        OWN ? make_double2(w[ki], __dmul_rn(w[ki], qinv))
+                        : R_LOG == 3
+                            ? __ldg(f.p + blk + (n + 1 - (n >> s) - skip + (uint32_t)ki * (n >> (s + 3))))
+                            : __ldg(f.p + (fp_inv_stage_index((blk << (R_LOG - t - 1)) + (k >> (t + 1)), s + t, LOGN) - skip));
                     v[k] = __dadd_rn(x, y);
                     v[k + h] = fp_mulmod(__dadd_rn(x, -y), m.x, m.y, q);
                 }
@@ -915,6 +913,158 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NttCfg<LOGB, V>::THR
     }
     cl.sync();
     for (int e = threadIdx.x; e < NB; e += T) op.store(c, e + off, sm[swz(e)]);
+}
+
+// ---------------------------------------------------------------- eight-CTA limbs
+// A whole limb of 2^(LOGB+3) coefficients on a cluster of eight CTAs, block r of 2^LOGB in
+// CTA r, a radix-8 group per thread and pass: for launches of so few limbs that even CTA
+// pairs leave most SMs idle (one ciphertext per call). One limb's butterflies then take an
+// eighth of an SM's time each instead of half. The three stages that join the blocks are
+// one radix-8 step through distributed shared memory: forward, CTA r loads the eight
+// operands of the groups j in its eighth of a block and stores each result into the block
+// it belongs to; inverse, it reads the eight blocks' words of its groups and stores the
+// results to global memory. One cluster barrier separates that step from the block's own
+// passes (and one before it makes sure that the CTAs have started, or keeps the shared
+// memory alive after it). In place is safe: every word is loaded before the barrier.
+constexpr int OCT_LOG = 3;
+template <int LOGB>
+struct OctCfg {
+    static constexpr int NB = 1 << LOGB;
+    static constexpr int THREADS = NB / 8;   // 64 .. 512
+};
+
+template <int LOGB, class Op>
+__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(OctCfg<LOGB>::THREADS) ntt_fwd_oct_kernel(Op op) {
+    extern __shared__ uint64_t sm[];
+    constexpr int NB = 1 << LOGB, T = OctCfg<LOGB>::THREADS, REM = LOGB % 3, LOGN = LOGB + OCT_LOG;
+    constexpr int FIRST = REM != 0 ? REM : 3;
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    cl.barrier_arrive();   // waited for before the first remote store
+    const unsigned r = cl.block_rank();
+    auto c = op.ctx((int)(blockIdx.x >> OCT_LOG));
+    c.lm.sb = r;
+    const int j = (int)r * T + (int)threadIdx.x, slot = swz(j);
+    if constexpr (LOGN >= FP_MIN_LOGN) {
+        if (c.lm.fp) {
+            double *smd = reinterpret_cast<double *>(sm);
+            const FpPass f{c.lm.fpm->w, c.lm.fpm->p, c.lm.fpm->q, c.lm.fpm->qinv, (c.lm.fp & FP_RED) != 0};
+            double v[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = fp_from_u64(op.load(c, j + (k << LOGB)));
+            fwd_group_fp<3>(
+                v, [&](int t, int k) { return __ldg(f.p + fp_fwd_stage_index(k + 1, t, LOGN)); }, f);
+            cl.barrier_wait();
+#pragma unroll
+            for (int k = 0; k < 8; k++) cl.map_shared_rank(smd, k)[slot] = v[k];
+            cl.sync();
+            ntt_fwd_block_fp<LOGB, T, OCT_LOG, false>(op, c, smd, f);
+            fwd_copy_out_fp<NB, T>(op, c, smd, (int)r << LOGB);
+            return;
+        }
+    }
+    {
+        const uint64_t q = c.lm.q, q2 = q << 1;
+        uint64_t v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = op.load(c, j + (k << LOGB));
+#pragma unroll
+        for (int t = 0; t < 3; t++) {
+            const int half = 8 >> (t + 1);
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                if (!(k & half)) ct_butterfly(v[k], v[k + half], __ldg(c.lm.roots + (1 << t) + (k >> (3 - t))), q, q2);
+        }
+        cl.barrier_wait();
+#pragma unroll
+        for (int k = 0; k < 8; k++) cl.map_shared_rank(sm, k)[slot] = v[k];
+    }
+    cl.sync();
+    const uint32_t rbase = 8u + r;   // global stage 3 onwards, sub-block = r
+    fwd_pass<FIRST, false, LOGB, T, 0, false>(op, c, sm, rbase);
+    fwd_passes<FIRST, LOGB, T, false>(op, c, sm, rbase);
+    fwd_copy_out<NB, T>(op, c, sm, (int)r << LOGB);
+}
+
+template <int LOGB, class Op>
+__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(OctCfg<LOGB>::THREADS) ntt_inv_oct_kernel(Op op) {
+    extern __shared__ uint64_t sm[];
+    constexpr int T = OctCfg<LOGB>::THREADS, REM = LOGB % 3, LOGN = LOGB + OCT_LOG;
+    constexpr uint32_t n = 1u << LOGN;
+    constexpr int LAST = REM ? REM : 3;
+    constexpr int PASSES = REM ? LOGB / 3 : LOGB / 3 - 1;
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const unsigned r = cl.block_rank();
+    auto c = op.ctx((int)(blockIdx.x >> OCT_LOG));
+    c.lm.sb = r;
+    const int j = (int)r * T + (int)threadIdx.x, slot = swz(j);
+    if constexpr (LOGN >= FP_MIN_LOGN) {
+        if (c.lm.fp) {
+            double *smd = reinterpret_cast<double *>(sm);
+            const FpPass f{c.lm.fpm->iw, c.lm.fpm->ip, c.lm.fpm->q, c.lm.fpm->qinv, (c.lm.fp & FP_RED) != 0};
+            const double q = f.q, qinv = f.qinv, si = c.lm.fpm->inv_n, sr = c.lm.fpm->sroot;
+            inv_copy_in<LOGB, T, true>(op, c, sm, (int)r << LOGB);
+            inv_passes_fp<0, PASSES, LOGB, T, LOGN>(op, c, smd, f);
+            inv_pass_fp<LAST, false, false, LOGB, T, 3 * PASSES, LOGN>(op, c, smd, f);
+            cl.sync();
+            double v[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = fp_reduce(cl.map_shared_rank(smd, k)[slot], q, qinv);
+            cl.barrier_arrive();   // this CTA is done with the others' shared memory
+#pragma unroll
+            for (int t = 0; t < 3; t++) {
+                const int h = 1 << t;
+                if (t == 2 && f.red) {
+                    v[0] = fp_reduce(v[0], q, qinv);
+                    v[4] = fp_reduce(v[4], q, qinv);
+                }
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    if (k & h) continue;
+                    const double x = v[k], y = v[k + h];
+                    if (t == 2) {
+                        v[k] = fp_mulmod(__dadd_rn(x, y), si, __dmul_rn(si, qinv), q);
+                        v[k + h] = fp_mulmod(__dadd_rn(x, -y), sr, __dmul_rn(sr, qinv), q);
+                    } else {
+                        const double w = __ldg(f.w + fp_inv_stage_index(k >> (t + 1), LOGB + t, LOGN));
+                        v[k] = __dadd_rn(x, y);
+                        v[k + h] = fp_mulmod(__dadd_rn(x, -y), w, __dmul_rn(w, qinv), q);
+                    }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) op.store(c, j + (k << LOGB), fp_to_residue(v[k], c.lm.q));
+            cl.barrier_wait();   // the others are done with this CTA's shared memory
+            return;
+        }
+    }
+    inv_copy_in<LOGB, T>(op, c, sm, (int)r << LOGB);
+    inv_passes<0, PASSES, LOGB, T, false>(op, c, sm, LOGN);
+    inv_pass<LAST, false, false, LOGB, T, 3 * PASSES, false>(op, c, sm, LOGN);
+    cl.sync();
+    const uint64_t q = c.lm.q, q2 = q << 1;
+    uint64_t v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = cl.map_shared_rank(sm, k)[slot];
+    cl.barrier_arrive();
+#pragma unroll
+    for (int t = 0; t < 3; t++) {
+        const int h = 1 << t;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            if (k & h) continue;
+            if (t == 2) {
+                const uint64_t u = csub(v[k], q2), y = v[k + h];
+                const uint64_t sum = csub(u + y, q2), dif = u + q2 - y;
+                v[k] = mul_shoup_lazy(sum, c.lm.inv_n, c.lm.inv_n_quo, q);
+                v[k + h] = mul_shoup_lazy(dif, c.lm.sroot, c.lm.sroot_quo, q);
+            } else {
+                gs_butterfly(v[k], v[k + h], __ldg(c.lm.iroots + (n + 1 - (n >> (LOGB + t)) + (k >> (t + 1)))), q, q2);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) op.store(c, j + (k << LOGB), v[k]);
+    cl.barrier_wait();
 }
 
 // ---------------------------------------------------------------- clusters of 4 and 8 CTAs
@@ -1160,6 +1310,21 @@ inline cudaError_t launch_cluster(const Op &op, unsigned blocks, cudaStream_t s)
     return cudaGetLastError();
 }
 
+// Whole limbs of 2^(LOGB+3) coefficients, eight CTAs each.
+template <bool FWD, int LOGB, class Op>
+inline cudaError_t launch_oct(const Op &op, unsigned blocks, cudaStream_t s) {
+    const size_t smem = ntt_smem_bytes<LOGB>();
+    static_assert(sizeof(uint64_t) << LOGB <= 48 * 1024, "no shared-memory opt-in");
+    if constexpr (FWD) ntt_fwd_oct_kernel<LOGB><<<8 * blocks, OctCfg<LOGB>::THREADS, smem, s>>>(op);
+    else ntt_inv_oct_kernel<LOGB><<<8 * blocks, OctCfg<LOGB>::THREADS, smem, s>>>(op);
+    return cudaGetLastError();
+}
+
+// Whether a launch of whole limbs takes the eight-CTA form: as many CTAs as two for every
+// SM at most. One pair of N = 8192 ciphertexts per call: mod-up 17 -> 11 us a launch, target
+// inverse 15 -> 11, mod-down 19 -> 13 (chain 166 -> 121 us).
+inline bool oct_launch(unsigned blocks) { return small_launch_pairs() && 4 * blocks <= (unsigned)sm_count(); }
+
 template <bool FWD, int LOGB, int V, class Op>
 inline cudaError_t launch_ntt(const Op &op, unsigned blocks, int s0_or_logn, int scale_last, cudaStream_t s) {
     if constexpr (V >= 3) {
@@ -1279,6 +1444,9 @@ cudaError_t dispatch_ntt(int logb, const Op &op, unsigned blocks, int s0_or_logn
         return launch_ntt<FWD, B, 0>(op, blocks, s0_or_logn, scale_last, s);
 #define TB_CASE2(B)                                                                  \
     case B:                                                                          \
+        if (ntt_variant(FWD, B) < 3 && oct_launch(blocks) &&                         \
+            (FWD ? s0_or_logn == 0 : (s0_or_logn == B && scale_last)))               \
+            return launch_oct<FWD, B - OCT_LOG>(op, blocks, s);                      \
         switch (large_launch_variant(small_launch_variant(ntt_variant(FWD, B), blocks), B, blocks)) { \
         case 1:                                                                      \
             return launch_ntt<FWD, B, 1>(op, blocks, s0_or_logn, scale_last, s);     \
@@ -1298,6 +1466,7 @@ cudaError_t dispatch_ntt(int logb, const Op &op, unsigned blocks, int s0_or_logn
         TB_CASE(8) TB_CASE(9) TB_CASE(10) TB_CASE(11) TB_CASE2(12) TB_CASE2(13) TB_CASE2(14)
     case PAIR_LOGN:
         if (FWD ? s0_or_logn != 0 : (s0_or_logn != PAIR_LOGN || !scale_last)) return cudaErrorInvalidValue;
+        if (oct_launch(blocks)) return launch_oct<FWD, PAIR_LOGN - OCT_LOG>(op, blocks, s);
         return launch_pair<FWD, MAX_LOGB, 0>(op, blocks, s);
     case MAX_LOGB + 2:
         if (FWD ? s0_or_logn != 0 : (s0_or_logn != MAX_LOGB + 2 || !scale_last)) return cudaErrorInvalidValue;
