@@ -206,20 +206,62 @@ struct ModUpOp {
     }
 };
 
+// acc += d k mod q for residues d, k below q < 2^50, exactly, up to a multiple of q: h + l
+// is the product, t the integer nearest h / q within 1/4 (h and 1 / q are rounded, h / q <
+// 2^50), so each term is an integer of at most 3/4 q. Seven FP64 instructions, where the
+// 128-bit multiply-accumulate takes about twelve issue slots of the FMA-heavy pipe.
+__device__ __forceinline__ void fp_mac(double &acc, double d, double k, double q, double qinv) {
+    const double h = __dmul_rn(d, k);
+    const double l = __fma_rn(d, k, -h);
+    const double t = __dadd_rn(__fma_rn(h, qinv, FP_ROUND), -FP_ROUND);
+    acc = __dadd_rn(acc, __dadd_rn(__fma_rn(-t, q, h), l));
+}
+
 // Step 3: acc[b][c][i] = sum_j digit(b, j, i) * key[j][c][mi] mod q_mi, two coefficients
-// (e, e+1) of output modulus i of ciphertext cb per thread.
+// (e, e+1) of output modulus i of ciphertext cb per thread. Moduli with an FP64 form have
+// canonical digits (their mod-up transforms run it) and take FP64 sums, reduced to q/2
+// every eight terms (below 7 q < 2^53).
 __device__ __forceinline__ void ks_inner_pair(const uint64_t *__restrict__ digits, const uint64_t *__restrict__ target,
                                               uint64_t tstride, const KeyGroups &keys, uint64_t *__restrict__ acc,
                                               const Mod *__restrict__ mods, int L, int K, int ckks, int logn,
                                               uint32_t e, int i, size_t cb) {
     const int mi = i == L ? K - 1 : i;
-    const Mod m = mods[mi];
     const uint64_t *__restrict__ key = keys.of((uint32_t)cb);
-    U128 a00{0, 0}, a01{0, 0}, a10{0, 0}, a11{0, 0};
     // running pointers: digit j of output modulus i, and key digit j (polys 0 and 1) at mi
     const size_t dstep = (size_t)(L + 1) << logn, kstep = (size_t)(2 * K) << logn, kpoly = (size_t)K << logn;
     const uint64_t *d = digits + ((cb * L * (L + 1) + i) << logn) + e;
     const uint64_t *k = key + ((size_t)mi << logn) + e;
+    uint64_t *o0 = acc + (((cb * 2 + 0) * (L + 1) + i) << logn) + e;
+    uint64_t *o1 = acc + (((cb * 2 + 1) * (L + 1) + i) << logn) + e;
+    if (const FpMod *f = mods[mi].fp) {
+        const double q = f->q, qinv = f->qinv;
+        double s00 = 0, s01 = 0, s10 = 0, s11 = 0;
+        for (int j = 0; j < L; j++, d += dstep, k += kstep) {
+            const uint64_t *dj = (ckks && i == j) ? target + cb * tstride + ((size_t)j << logn) + e : d;
+            const ulonglong2 dv = *reinterpret_cast<const ulonglong2 *>(dj);
+            const ulonglong2 k0 = __ldg(reinterpret_cast<const ulonglong2 *>(k));
+            const ulonglong2 k1 = __ldg(reinterpret_cast<const ulonglong2 *>(k + kpoly));
+            const double dx = fp_from_u64(dv.x), dy = fp_from_u64(dv.y);
+            fp_mac(s00, dx, fp_from_u64(k0.x), q, qinv);
+            fp_mac(s01, dy, fp_from_u64(k0.y), q, qinv);
+            fp_mac(s10, dx, fp_from_u64(k1.x), q, qinv);
+            fp_mac(s11, dy, fp_from_u64(k1.y), q, qinv);
+            if ((j & 7) == 7) {
+                s00 = fp_reduce(s00, q, qinv);
+                s01 = fp_reduce(s01, q, qinv);
+                s10 = fp_reduce(s10, q, qinv);
+                s11 = fp_reduce(s11, q, qinv);
+            }
+        }
+        const uint64_t qi = mods[mi].value;
+        *reinterpret_cast<ulonglong2 *>(o0) =
+            make_ulonglong2(fp_to_residue(fp_reduce(s00, q, qinv), qi), fp_to_residue(fp_reduce(s01, q, qinv), qi));
+        *reinterpret_cast<ulonglong2 *>(o1) =
+            make_ulonglong2(fp_to_residue(fp_reduce(s10, q, qinv), qi), fp_to_residue(fp_reduce(s11, q, qinv), qi));
+        return;
+    }
+    const Mod m = mods[mi];
+    U128 a00{0, 0}, a01{0, 0}, a10{0, 0}, a11{0, 0};
     for (int j = 0; j < L; j++, d += dstep, k += kstep) {
         const uint64_t *dj = (ckks && i == j) ? target + cb * tstride + ((size_t)j << logn) + e : d;
         const ulonglong2 dv = *reinterpret_cast<const ulonglong2 *>(dj);
@@ -230,8 +272,6 @@ __device__ __forceinline__ void ks_inner_pair(const uint64_t *__restrict__ digit
         mac128(a10, dv.x, k1.x);
         mac128(a11, dv.y, k1.y);
     }
-    uint64_t *o0 = acc + (((cb * 2 + 0) * (L + 1) + i) << logn) + e;
-    uint64_t *o1 = acc + (((cb * 2 + 1) * (L + 1) + i) << logn) + e;
     *reinterpret_cast<ulonglong2 *>(o0) = make_ulonglong2(reduce128(a00.hi, a00.lo, m), reduce128(a01.hi, a01.lo, m));
     *reinterpret_cast<ulonglong2 *>(o1) = make_ulonglong2(reduce128(a10.hi, a10.lo, m), reduce128(a11.hi, a11.lo, m));
 }
