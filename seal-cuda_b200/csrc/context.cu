@@ -169,7 +169,9 @@ int context_create(int scheme, uint64_t n, const uint64_t *moduli, int count, ui
         for (auto p : extra) c->table_moduli.push_back(p);
     }
     const size_t nm = c->table_moduli.size();
-    std::vector<ulonglong2> all(2 * nm * n);
+    // per modulus: forward and inverse twiddles, and both again in the order of the radix-8
+    // passes (fp64mod.cuh), 2 N further on
+    std::vector<ulonglong2> all(4 * nm * n);
     c->h_mods.resize(nm);
     for (size_t i = 0; i < nm; i++) {
         std::vector<ulonglong2> f, v;
@@ -177,8 +179,15 @@ int context_create(int scheme, uint64_t n, const uint64_t *moduli, int count, ui
             delete c;
             return set_error(TB_ERR_INVALID_ARGUMENT, "modulus has no primitive 2N-th root of unity");
         }
-        std::memcpy(&all[(2 * i) * n], f.data(), n * sizeof(ulonglong2));
-        std::memcpy(&all[(2 * i + 1) * n], v.data(), n * sizeof(ulonglong2));
+        ulonglong2 *t = &all[4 * i * n];
+        std::memcpy(t, f.data(), n * sizeof(ulonglong2));
+        std::memcpy(t + n, v.data(), n * sizeof(ulonglong2));
+        t[2 * n] = f[0];
+        t[3 * n] = v[0];
+        for (uint32_t k = 1; k < n; k++) {
+            t[2 * n + fp_fwd_index(k, c->logn)] = f[k];
+            t[3 * n + fp_inv_index(k, c->logn)] = v[k];
+        }
     }
     cudaError_t e = cudaMalloc(&c->d_tables, all.size() * sizeof(ulonglong2));
     if (e == cudaSuccess) e = cudaMemcpy(c->d_tables, all.data(), all.size() * sizeof(ulonglong2), cudaMemcpyHostToDevice);
@@ -187,8 +196,8 @@ int context_create(int scheme, uint64_t n, const uint64_t *moduli, int count, ui
         return status_from(e);
     }
     for (size_t i = 0; i < nm; i++) {
-        c->h_mods[i].roots = c->d_tables + (2 * i) * n;
-        c->h_mods[i].inv_roots = c->d_tables + (2 * i + 1) * n;
+        c->h_mods[i].roots = c->d_tables + 4 * i * n;
+        c->h_mods[i].inv_roots = c->d_tables + (4 * i + 1) * n;
     }
     e = build_fp_tables(*c);
     if (e == cudaSuccess) e = cudaMalloc(&c->d_mods, nm * sizeof(Mod));
@@ -212,6 +221,7 @@ int context_create(int scheme, uint64_t n, const uint64_t *moduli, int count, ui
 // [polys][limbs][n] in -> out; a CTA owns one limb, or one 2^LOGB sub-block of it.
 template <bool FWD>
 struct PlainNttOp {
+    static constexpr bool sub_blocks = true;   // CTAs of longer limbs
     const uint64_t *in;
     uint64_t *out;
     const Mod *mods;

@@ -69,9 +69,10 @@ __device__ __forceinline__ double fp_centred(uint64_t w, uint64_t q) {
     return w > (q >> 1) ? -fp_from_u64(q - w) : fp_from_u64(w);
 }
 
-// Where the FP64 tables keep the twiddles of the integer tables. The three stages of a
+// Where the pass-ordered tables (FP64, and the integer ones at roots + 2 N) keep the
+// twiddles of the integer tables in natural order. The three stages of a
 // radix-8 pass starting at stage s use 7 consecutive ranges of 2^s twiddles (forward:
-// indices 2^s .. 8 2^s - 1); the FP64 tables hold, inside the same range, twiddle k (0 ..
+// indices 2^s .. 8 2^s - 1); the ordered tables hold, inside the same range, twiddle k (0 ..
 // 6, in stage order) of every group side by side, so a warp's loads of one k are
 // consecutive. Radix-8 passes end at the last stage, so the stages before the first one
 // (logn mod 3) keep their natural order. index 1 .. n - 1.
