@@ -49,6 +49,7 @@ struct RnsOff {
     int B_ip;          // pair[bB]: (P_B/B_k)^-1 mod B_k
     int tq_ip;         // pair[L]: t (Q/q_i)^-1 mod q_i
     int iqb_Bip;       // pair[bB]: Q^-1 (P_B/B_k)^-1 mod B_k (c_k of B_k; c of m_sk is Q^-1)
+    int M_qB_s;        // [bsk][L]: the lift rows, each word split in 30-bit halves (multiply.cu)
     int M_Bq;          // [L][bB]: (P_B/B_k) mod q_i
     int M_Bmsk;        // [bB]: (P_B/B_k) mod m_sk
     int inv_pb_msk;    // pair: P_B^-1 mod m_sk
@@ -71,6 +72,7 @@ struct RnsOff {
 struct RnsLevel {
     int L = 0;                  // data limbs at this level (moduli chain[0..L-1])
     int bB = 0, bsk = 0;        // |B| and |Bsk| = |B| + 1
+    bool split = false;         // the lift kernel's split sums apply (all q_i below 2^58, L <= 16)
     uint64_t m_sk = 0, gamma = 0;
     RnsOff off{};
     uint64_t *d_consts = nullptr;

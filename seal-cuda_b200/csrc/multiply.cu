@@ -71,6 +71,7 @@ int build_level_consts(Context &c, int L) {
     o.B_ip = take(2 * bB);
     o.tq_ip = take(2 * L);
     o.iqb_Bip = take(2 * bB);
+    o.M_qB_s = take(bsk * L);
     o.M_Bq = take(L * bB);
     o.M_Bmsk = take(bB);
     o.inv_pb_msk = take(2);
@@ -159,6 +160,11 @@ int build_level_consts(Context &c, int L) {
         pair(o.cdpt, i, mod_words(Qdt, q[i]), q[i]);
         h[o.plain_incr + i] = (q[i] - t % q[i]) % q[i];
     }
+    // split forms: low 30 bits in the low word, the rest in the high word
+    auto split = [](uint64_t v) { return (v & ((1u << 30) - 1)) | (v >> 30) << 32; };
+    for (int i = 0; i < bsk * L; i++) h[o.M_qB_s + i] = split(h[o.M_qB + i]);
+    lv.split = L <= 16;
+    for (int i = 0; i < L; i++) lv.split &= q[i] < (1ull << 58);
     if (!ok) return TB_OK;  // t shares a factor with q: BFV/BGV arithmetic unavailable at this level
     std::vector<Mod> bm(bsk);
     for (int k = 0; k < bsk; k++) bm[k] = c.h_mods[bidx[k]];
@@ -189,10 +195,55 @@ __device__ __forceinline__ uint64_t pw(const uint64_t *K, int off, int i, uint64
 // registers; the loops over the B / Bsk primes stay rolled, so one iteration's constants
 // are all that is live beside them.
 
+// The lift's base-conversion sums from 30-bit halves (SPLIT, for q_i < 2^58 and at most 16
+// limbs). The 64x64-bit multiply-accumulate into 128 bits takes about 14 issue slots of the
+// FMA-heavy pipe (one low and one high 64-bit product); x = x0 + 2^30 x1 and c = c0 + 2^30
+// c1 take four 32x32-bit multiply-adds into three 64-bit sums without carries, 8 slots. x is
+// below 2^58 and c below 2^61, so a term adds less than 2^60, 2^61 + 2^58 and 2^59 to the
+// sums: seven terms fit, then they are folded into a 128-bit sum, below 16 * 2^58 * 2^61 =
+// 2^123 in the end, reduce_prod's range for a 61-bit modulus (one quotient product instead
+// of three). 192 polynomials of N = 16384, L = 8: 373 -> 337 us. In the floor kernel, whose
+// registers are full, the same sums gained 2% and are not used.
+constexpr int FOLD = 7;
+struct Acc3 {
+    uint64_t lo = 0, mid = 0, hi = 0;
+};
+struct Halves {
+    uint32_t lo, hi;
+};
+__device__ __forceinline__ Halves halves(uint64_t x) { return {(uint32_t)x & ((1u << 30) - 1), (uint32_t)(x >> 30)}; }
+__device__ __forceinline__ void mac3(Acc3 &a, Halves x, uint64_t c) {
+    const uint32_t c0 = (uint32_t)c, c1 = (uint32_t)(c >> 32);
+    a.lo += (uint64_t)x.lo * c0;
+    a.mid += (uint64_t)x.lo * c1;
+    a.mid += (uint64_t)x.hi * c0;
+    a.hi += (uint64_t)x.hi * c1;
+}
+__device__ __forceinline__ void fold(U128 &s, Acc3 &a) {
+    const unsigned __int128 v = (unsigned __int128)a.lo + ((unsigned __int128)a.mid << 30) + ((unsigned __int128)a.hi << 60) +
+                                (((unsigned __int128)s.hi << 64) | s.lo);
+    s.lo = (uint64_t)v;
+    s.hi = (uint64_t)(v >> 64);
+    a = Acc3();
+}
+
+// sum_i x_i c_i mod m over the NL = LT data limbs (split words and constants).
+template <int LT>
+__device__ __forceinline__ uint64_t split_sum(const Halves *x, const uint64_t *c, const Mod &m) {
+    U128 s{0, 0};
+    Acc3 a;
+#pragma unroll
+    for (int i = 0; i < LT; i++) {
+        mac3(a, x[i], c[i]);
+        if (i % FOLD == FOLD - 1 || i == LT - 1) fold(s, a);
+    }
+    return reduce_prod(s.hi, s.lo, m);
+}
+
 // Steps (1)+(2): q (coefficient form) -> Bsk, one coefficient per thread, for both
 // inputs of B products: polynomial p = ct*4 + slot, slots 0,1 from a and 2,3 from b;
 // output [B][4][bsk][N].
-template <int LT>
+template <int LT, bool SPLIT = false>
 __global__ void __launch_bounds__(256, 3) behz_lift_kernel(const uint64_t *__restrict__ a, uint64_t astride,
                                                         const uint64_t *__restrict__ b, uint64_t bstride,
                                                         uint64_t *__restrict__ dst, const Mod *__restrict__ qm,
@@ -218,16 +269,26 @@ __global__ void __launch_bounds__(256, 3) behz_lift_kernel(const uint64_t *__res
         }
         const uint64_t r = ((mt & 0xffffffffull) * K[o.neg_inv_q_mt]) & 0xffffffffull;
         uint64_t *out = dst + ((p * bsk) << logn) + e;
+        Halves x[SPLIT ? NL : 1];
+        if constexpr (SPLIT) {
+#pragma unroll
+            for (int i = 0; i < NL; i++) x[i] = halves(tmp[i]);
+        }
 #pragma unroll 1
         for (int k = 0; k < bsk; k++) {
             const Mod &m = bm[k];
-            U128 acc{0, 0};
+            uint64_t v;   // already times m~^-1
+            if constexpr (SPLIT) {
+                v = split_sum<LT>(x, K + o.M_qB_s + k * LT, m);
+            } else {
+                U128 acc{0, 0};
 #pragma unroll UNROLL
-            for (int i = 0; i < NL; i++) {
-                if (i >= L) break;
-                mac128(acc, tmp[i], K[o.M_qB + k * L + i]);
+                for (int i = 0; i < NL; i++) {
+                    if (i >= L) break;
+                    mac128(acc, tmp[i], K[o.M_qB + k * L + i]);
+                }
+                v = reduce128(acc.hi, acc.lo, m);
             }
-            const uint64_t v = reduce128(acc.hi, acc.lo, m);   // already times m~^-1
             const uint64_t rr = r >= (1ull << 31) ? r + m.value - (1ull << 32) : r;
             out[(size_t)k << logn] = add_mod(pw(K, o.Qmt_b, k, rr, m.value), v, m.value);
         }
@@ -309,8 +370,9 @@ __global__ void __launch_bounds__(256, 2) behz_floor_sk_kernel(const uint64_t *_
 template <int LT>
 struct LiftLaunch {
     template <class... A>
-    static cudaError_t run(uint64_t threads, cudaStream_t s, A... args) {
-        behz_lift_kernel<LT><<<grid_for(threads, 256), 256, 0, s>>>(args...);
+    static cudaError_t run(bool split, uint64_t threads, cudaStream_t s, A... args) {
+        auto k = split && LT > 0 ? behz_lift_kernel<LT, (LT > 0)> : behz_lift_kernel<LT>;
+        k<<<grid_for(threads, 256), 256, 0, s>>>(args...);
         return cudaGetLastError();
     }
 };
@@ -318,7 +380,7 @@ struct LiftLaunch {
 template <int LT>
 struct FloorLaunch {
     template <class... A>
-    static cudaError_t run(uint64_t threads, cudaStream_t s, A... args) {
+    static cudaError_t run(bool, uint64_t threads, cudaStream_t s, A... args) {
         behz_floor_sk_kernel<LT><<<grid_for(threads, 256), 256, 0, s>>>(args...);
         return cudaGetLastError();
     }
@@ -328,16 +390,16 @@ struct FloorLaunch {
 // up to 32 limbs and its wide form above.
 #define TB_BEHZ_CASE(LV) \
     case LV:             \
-        return Launch<LV>::run(threads, s, args...);
+        return Launch<LV>::run(split, threads, s, args...);
 template <template <int> class Launch, class... A>
-cudaError_t behz_dispatch(int L, uint64_t threads, cudaStream_t s, A... args) {
+cudaError_t behz_dispatch(int L, bool split, uint64_t threads, cudaStream_t s, A... args) {
     switch (L) {
         TB_BEHZ_CASE(1) TB_BEHZ_CASE(2) TB_BEHZ_CASE(3) TB_BEHZ_CASE(4) TB_BEHZ_CASE(5) TB_BEHZ_CASE(6)
         TB_BEHZ_CASE(7) TB_BEHZ_CASE(8) TB_BEHZ_CASE(9) TB_BEHZ_CASE(10) TB_BEHZ_CASE(11) TB_BEHZ_CASE(12)
         TB_BEHZ_CASE(13) TB_BEHZ_CASE(14) TB_BEHZ_CASE(15) TB_BEHZ_CASE(16)
     default:
-        if (L <= MAXL_RT) return Launch<0>::run(threads, s, args...);
-        return Launch<-1>::run(threads, s, args...);
+        if (L <= MAXL_RT) return Launch<0>::run(split, threads, s, args...);
+        return Launch<-1>::run(split, threads, s, args...);
     }
 }
 #undef TB_BEHZ_CASE
@@ -490,6 +552,10 @@ int multiply(const Context &c, int L, const uint64_t *a, uint64_t astride, const
     ensure_pool_retains(c.device);
     const int logn = c.logn;
     cudaError_t e;
+    // FP64 transforms give canonical words: the tensor's one-product reduction applies
+    // (making the integer forms' words canonical in their stores cost more than it saved)
+    bool canon = true;
+    for (int l = 0; l < L; l++) canon = canon && c.h_mods[l].fp;
     if (c.scheme == SCHEME_BGV) {
         ScratchBuf buf(s);
         e = cudaMallocAsync(&buf.p, B * 7ull * L * n * 8, s);
@@ -502,7 +568,7 @@ int multiply(const Context &c, int L, const uint64_t *a, uint64_t astride, const
         }
         if (e != cudaSuccess) return status_from(e);
         const uint64_t pq = (uint64_t)L * n;
-        int st = tensor_product_mods(c, c.d_mods, L, x, 4 * pq, x + 2 * pq, 4 * pq, tn, 3 * pq, B, s);
+        int st = tensor_product_mods(c, c.d_mods, L, x, 4 * pq, x + 2 * pq, 4 * pq, tn, 3 * pq, B, s, canon);
         if (st != TB_OK) return st;
         TraceScope ts("mul_intt", s);
         CtInttOutOp oi{tn, out, ostride, c.d_mods, 3, L, logn};
@@ -518,7 +584,7 @@ int multiply(const Context &c, int L, const uint64_t *a, uint64_t astride, const
     ScratchBuf buf(s);
     e = cudaMallocAsync(&buf.p, B * (4 * pq + 4 * pb + 3 * pq + 3 * pb) * 8, s);
     if (e != cudaSuccess) return status_from(e);
-    uint64_t *xq = (uint64_t *)buf.p;          // [B][4][L][N]: a0 a1 b0 b1 (NTT, lazy)
+    uint64_t *xq = (uint64_t *)buf.p;          // [B][4][L][N]: a0 a1 b0 b1 (NTT)
     uint64_t *xb = xq + B * 4 * pq;            // [B][4][bsk][N]
     uint64_t *tq = xb + B * 4 * pb;            // [B][3][L][N]
     uint64_t *tbk = tq + B * 3 * pq;           // [B][3][bsk][N]
@@ -530,7 +596,7 @@ int multiply(const Context &c, int L, const uint64_t *a, uint64_t astride, const
     }
     {
         TraceScope ts("bfv_lift", s);
-        e = behz_dispatch<LiftLaunch>(L, 4 * B * n, s, a, astride, b, bstride, xb, (const Mod *)c.d_mods,
+        e = behz_dispatch<LiftLaunch>(L, lv.split, 4 * B * n, s, a, astride, b, bstride, xb, (const Mod *)c.d_mods,
                                       (const Mod *)lv.d_bsk_mods, (const uint64_t *)lv.d_consts, lv.off, L, bsk, logn,
                                       (uint64_t)(4 * B));
         if (e != cudaSuccess) return status_from(e);
@@ -541,7 +607,7 @@ int multiply(const Context &c, int L, const uint64_t *a, uint64_t astride, const
         e = dispatch_ntt<true>(logn, op, (unsigned)(B * 4 * bsk), 0, 0, s);
         if (e != cudaSuccess) return status_from(e);
     }
-    int st = tensor_product_mods(c, c.d_mods, L, xq, 4 * pq, xq + 2 * pq, 4 * pq, tq, 3 * pq, B, s);
+    int st = tensor_product_mods(c, c.d_mods, L, xq, 4 * pq, xq + 2 * pq, 4 * pq, tq, 3 * pq, B, s, canon);
     if (st != TB_OK) return st;
     st = tensor_product_mods(c, lv.d_bsk_mods, bsk, xb, 4 * pb, xb + 2 * pb, 4 * pb, tbk, 3 * pb, B, s);
     if (st != TB_OK) return st;
@@ -556,7 +622,7 @@ int multiply(const Context &c, int L, const uint64_t *a, uint64_t astride, const
     }
     {
         TraceScope ts("bfv_floor_sk", s);
-        e = behz_dispatch<FloorLaunch>(L, 3 * B * n, s, (const uint64_t *)tq, (const uint64_t *)tbk, out, ostride,
+        e = behz_dispatch<FloorLaunch>(L, lv.split, 3 * B * n, s, (const uint64_t *)tq, (const uint64_t *)tbk, out, ostride,
                                        (const Mod *)c.d_mods, (const Mod *)lv.d_bsk_mods, (const uint64_t *)lv.d_consts,
                                        lv.off, L, lv.bB, logn, (uint64_t)(3 * B));
     }
@@ -646,7 +712,7 @@ int multiply_sizes(const Context &c, int L, const uint64_t *a, int sa, const uin
     if (e != cudaSuccess) return status_from(e);
     // the lift reads polynomial p of four-polynomial groups: with both strides 4 L N
     // and b starting two polynomials in, polynomial p of x0 for every p
-    e = behz_dispatch<LiftLaunch>(L, (uint64_t)P * n, s, (const uint64_t *)x0, 4 * pq,
+    e = behz_dispatch<LiftLaunch>(L, lv.split, (uint64_t)P * n, s, (const uint64_t *)x0, 4 * pq,
                                   (const uint64_t *)(x0 + 2 * pq), 4 * pq, xb, (const Mod *)c.d_mods,
                                   (const Mod *)lv.d_bsk_mods, (const uint64_t *)lv.d_consts, lv.off, L, bsk, logn,
                                   (uint64_t)P);
@@ -666,7 +732,7 @@ int multiply_sizes(const Context &c, int L, const uint64_t *a, int sa, const uin
     e = dispatch_ntt<false>(logn, ib, (unsigned)(D * bsk), logn, 1, s);
     if (e != cudaSuccess) return status_from(e);
     // the floor reads polynomial p = ct * 3 + poly: ostride 3 L N maps it to out + p L N
-    e = behz_dispatch<FloorLaunch>(L, (uint64_t)D * n, s, (const uint64_t *)tq, (const uint64_t *)tbk, out,
+    e = behz_dispatch<FloorLaunch>(L, lv.split, (uint64_t)D * n, s, (const uint64_t *)tq, (const uint64_t *)tbk, out,
                                    3 * pq, (const Mod *)c.d_mods, (const Mod *)lv.d_bsk_mods,
                                    (const uint64_t *)lv.d_consts, lv.off, L, lv.bB, logn, (uint64_t)D);
     return status_from(e);
