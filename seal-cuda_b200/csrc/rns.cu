@@ -72,7 +72,7 @@ struct LastInttOp {
     __device__ Ctx ctx(int b) const {
         Ctx c;
         c.lm = make_limb(mods[L - 1], 0);
-        c.lm.fp = fp_form(mods[L - 1]);
+        c.lm.fp = fp_form(mods[L - 1], true);   // any words below 4 q, as the wide form
         c.in = in + (size_t)(b / size) * istride + ((size_t)((b % size) * L + L - 1) << logn);
         c.out = r + ((size_t)b << logn);
         c.islack = 1;
