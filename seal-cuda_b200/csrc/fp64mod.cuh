@@ -42,9 +42,6 @@ __device__ __forceinline__ double fp_from_u64(uint64_t x) {
     return __dadd_rn(__longlong_as_double((long long)(x | 0x4330000000000000ull)), -FP_2P52);
 }
 
-// The integer nearest x for |x| < 2^51.
-__device__ __forceinline__ double fp_rint(double x) { return __dadd_rn(__dadd_rn(x, FP_ROUND), -FP_ROUND); }
-
 __device__ __forceinline__ double fp_mulmod(double y, double w, double wq, double q) {
     const double t = __dadd_rn(__fma_rn(y, wq, FP_ROUND), -FP_ROUND);
     const double h = __dmul_rn(y, w);

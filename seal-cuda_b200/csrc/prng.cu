@@ -5,7 +5,7 @@
 // little-endian counter 0, 1, 2, ... as message. That makes the stream counter
 // based: byte p lives in refill p / 4096, output block (p % 4096) / 64, and every
 // 64-byte block is one BLAKE2b compression of the refill's root hash. prng_fill
-// computes any byte range in parallel (one thread per 64-byte block; BLAKE2b as in
+// computes any byte range in parallel (four lanes per 64-byte block; BLAKE2b as in
 // RFC 7693, BLAKE2X parameters per the BLAKE2X specification).
 //
 // A PRNG is a device-resident PrngState {seed, offset}: samplers read the offset,

@@ -18,7 +18,7 @@ SEEDP = (ctypes.c_uint64 * 8)(*[int(x) for x in SEED])
 
 
 def _dev(a):
-    return torch.from_numpy(np.array(a, np.uint64).view(np.int64)).cuda()
+    return torch.from_numpy(np.array(a, np.uint64, order="C").view(np.int64)).cuda()
 
 
 def _host(t):
