@@ -429,7 +429,8 @@ static int ckks_tables(Context &c, double2 **roots, double2 **iroots) {
             if (idx <= 3 * m / 4) return -get(idx - m / 2);
             return std::conj(get(m - idx));
         };
-        std::vector<double2> r(n, make_double2(0, 0)), ir(n, make_double2(0, 0));
+        std::vector<double2> r(2ull * n, make_double2(0, 0));   // forward, inverse
+        double2 *ir = r.data() + n;
         if (m >= 8) {
             for (uint32_t i = 1; i < n; i++) {
                 auto a = get(host::bitrev(i, c.logn));
@@ -442,9 +443,7 @@ static int ckks_tables(Context &c, double2 **roots, double2 **iroots) {
             ir[1] = make_double2(0, -1);
         }
         double2 *d = nullptr;
-        cudaError_t e = cudaMalloc(&d, 2ull * n * sizeof(double2));
-        if (e == cudaSuccess) e = cudaMemcpy(d, r.data(), n * sizeof(double2), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(d + n, ir.data(), n * sizeof(double2), cudaMemcpyHostToDevice);
+        const cudaError_t e = to_device(r.data(), r.size(), &d);
         if (e != cudaSuccess) return status_from(e);
         c.d_fft_roots = d;
     }
@@ -636,14 +635,8 @@ static int compose_consts(Context &c, int L, const uint64_t **out) {
             carry = v & 1;
         }
         for (int i = 0; i < L; i++) hc[2 * L + L * L + L + i] = t[i];
-        uint64_t *d = nullptr;
-        cudaError_t e = cudaMalloc(&d, hc.size() * 8);
-        if (e == cudaSuccess) e = cudaMemcpy(d, hc.data(), hc.size() * 8, cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) {
-            if (d) cudaFree(d);
-            return status_from(e);
-        }
-        lv.d_compose = d;
+        const cudaError_t e = to_device(hc.data(), hc.size(), &lv.d_compose);
+        if (e != cudaSuccess) return status_from(e);
     }
     *out = lv.d_compose;
     return TB_OK;

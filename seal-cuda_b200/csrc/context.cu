@@ -189,8 +189,7 @@ int context_create(int scheme, uint64_t n, const uint64_t *moduli, int count, ui
             t[3 * n + fp_inv_index(k, c->logn)] = v[k];
         }
     }
-    cudaError_t e = cudaMalloc(&c->d_tables, all.size() * sizeof(ulonglong2));
-    if (e == cudaSuccess) e = cudaMemcpy(c->d_tables, all.data(), all.size() * sizeof(ulonglong2), cudaMemcpyHostToDevice);
+    cudaError_t e = to_device(all.data(), all.size(), &c->d_tables);
     if (e != cudaSuccess) {
         delete c;
         return status_from(e);
@@ -200,8 +199,7 @@ int context_create(int scheme, uint64_t n, const uint64_t *moduli, int count, ui
         c->h_mods[i].inv_roots = c->d_tables + (4 * i + 1) * n;
     }
     e = build_fp_tables(*c);
-    if (e == cudaSuccess) e = cudaMalloc(&c->d_mods, nm * sizeof(Mod));
-    if (e == cudaSuccess) e = cudaMemcpy(c->d_mods, c->h_mods.data(), nm * sizeof(Mod), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = to_device(c->h_mods.data(), nm, &c->d_mods);
     if (e != cudaSuccess) {
         delete c;
         return status_from(e);

@@ -31,6 +31,21 @@ int set_error(int status, const std::string &msg);
 // The status of a call that does not run inside a stream capture (TB_OK outside one).
 int refuse_capture(cudaStream_t s);
 
+// Device copy (cudaMalloc) of `count` items of a table that outlives the call, for kernels
+// on any stream from then on: a pageable cudaMemcpy may return before its data is on the
+// device, and a non-blocking stream is not ordered after the legacy one, so the copy is
+// waited for here. *out is set on success only.
+template <class T>
+cudaError_t to_device(const T *src, size_t count, T **out) {
+    T *d = nullptr;
+    cudaError_t e = cudaMalloc(&d, count * sizeof(T));
+    if (e == cudaSuccess) e = cudaMemcpy(d, src, count * sizeof(T), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    if (e == cudaSuccess) *out = d;
+    else if (d) cudaFree(d);
+    return e;
+}
+
 // Offsets (in words) of the per-level RNS constants inside RnsLevel::d_consts.
 // "pair" entries are Shoup operands stored as consecutive {operand, quotient}.
 struct RnsOff {

@@ -912,12 +912,8 @@ int galois_ntt_table(Context &c, uint32_t elt, const uint32_t **out) {
         t[i] = host::bitrev((uint32_t)raw, c.logn);
     }
     uint32_t *d = nullptr;
-    cudaError_t e = cudaMalloc(&d, n * 4);
-    if (e == cudaSuccess) e = cudaMemcpy(d, t.data(), n * 4, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-        if (d) cudaFree(d);
-        return status_from(e);
-    }
+    const cudaError_t e = to_device(t.data(), n, &d);
+    if (e != cudaSuccess) return status_from(e);
     c.galois_ntt[elt] = d;
     *out = d;
     return TB_OK;

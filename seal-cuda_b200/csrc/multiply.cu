@@ -168,12 +168,9 @@ int build_level_consts(Context &c, int L) {
     if (!ok) return TB_OK;  // t shares a factor with q: BFV/BGV arithmetic unavailable at this level
     std::vector<Mod> bm(bsk);
     for (int k = 0; k < bsk; k++) bm[k] = c.h_mods[bidx[k]];
-    cudaError_t e = cudaMalloc(&lv.d_consts, h.size() * 8);
-    if (e == cudaSuccess) e = cudaMemcpy(lv.d_consts, h.data(), h.size() * 8, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMalloc(&lv.d_bsk_mods, bsk * sizeof(Mod));
-    if (e == cudaSuccess) e = cudaMemcpy(lv.d_bsk_mods, bm.data(), bsk * sizeof(Mod), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMalloc(&lv.d_bsk_idx, bsk * sizeof(int));
-    if (e == cudaSuccess) e = cudaMemcpy(lv.d_bsk_idx, bidx.data(), bsk * sizeof(int), cudaMemcpyHostToDevice);
+    cudaError_t e = to_device(h.data(), h.size(), &lv.d_consts);
+    if (e == cudaSuccess) e = to_device(bm.data(), bsk, &lv.d_bsk_mods);
+    if (e == cudaSuccess) e = to_device(bidx.data(), bsk, &lv.d_bsk_idx);
     return e == cudaSuccess ? TB_OK : status_from(e);
 }
 

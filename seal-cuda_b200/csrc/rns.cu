@@ -33,8 +33,7 @@ int build_rns_levels(Context &c) {
             drop[(size_t)Lf * K + j] = d;
         }
     }
-    cudaError_t e = cudaMalloc(&c.d_drop, drop.size() * sizeof(DropC));
-    if (e == cudaSuccess) e = cudaMemcpy(c.d_drop, drop.data(), drop.size() * sizeof(DropC), cudaMemcpyHostToDevice);
+    cudaError_t e = to_device(drop.data(), drop.size(), &c.d_drop);
     if (e != cudaSuccess) return status_from(e);
     if (c.t) {
         c.t_mod.value = c.t;

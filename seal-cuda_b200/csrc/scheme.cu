@@ -648,11 +648,7 @@ int slot_map(Context &c, const uint32_t **out) {
         // the map (slot -> coefficient) and its inverse
         map.resize(2 * n);
         for (uint32_t i = 0; i < n; i++) map[n + map[i]] = i;
-        uint32_t *d = nullptr;
-        cudaError_t e = cudaMalloc(&d, 2ull * n * 4);
-        if (e == cudaSuccess) e = cudaMemcpy(d, map.data(), 2ull * n * 4, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) c.d_slot_map = d;
-        else if (d) cudaFree(d);
+        const cudaError_t e = to_device(map.data(), map.size(), &c.d_slot_map);
         if (e != cudaSuccess) return status_from(e);
     }
     *out = c.d_slot_map;
