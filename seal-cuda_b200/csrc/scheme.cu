@@ -1015,7 +1015,9 @@ int batch_encode(Context &c, const uint64_t *slots, uint64_t sstride, uint32_t c
     return status_from(dispatch_ntt<false>(c.logn, op, (unsigned)B, c.logn, 1, s));
 }
 
-// plaintexts [B][N] -> slots [B][N] (BatchEncoder::decode).
+// plaintexts [B][N] -> slots [B][N] (BatchEncoder::decode). Slots may overlap plaintexts:
+// the limbs of a launch run in any order, so unless every plaintext is replaced by its own
+// slots, overlapped plaintexts are read from a copy.
 int batch_decode(Context &c, const uint64_t *plain, uint64_t *slots, uint64_t sstride, uint64_t B, cudaStream_t s) {
     if (c.plain_index < 0) return set_error(TB_ERR_UNSUPPORTED, "plain modulus does not support batching");
     if (!plain || !slots) return set_error(TB_ERR_INVALID_ARGUMENT, "null buffer");
@@ -1025,6 +1027,14 @@ int batch_decode(Context &c, const uint64_t *plain, uint64_t *slots, uint64_t ss
     int r = slot_map(c, &map);
     if (r != TB_OK) return r;
     if (B > 0x7fffffffull) return set_error(TB_ERR_INVALID_ARGUMENT, "too many plaintexts in one call");
+    const bool overlap = slots < plain + B * c.n && plain < slots + (B - 1) * sstride + c.n;
+    DevBuf tmp(s);
+    if (overlap && !(slots == plain && sstride == c.n)) {
+        cudaError_t e = tmp.alloc(8ull * B * c.n);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(tmp.p, plain, 8ull * B * c.n, cudaMemcpyDeviceToDevice, s);
+        if (e != cudaSuccess) return status_from(e);
+        plain = tmp.as<uint64_t>();
+    }
     TraceScope ts("batch_decode", s);
     BatchDecodeOp op{plain, slots, sstride, map + c.n, c.d_mods + c.plain_index, c.logn};
     return status_from(dispatch_ntt<true>(c.logn, op, (unsigned)B, 0, 0, s));

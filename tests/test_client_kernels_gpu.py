@@ -172,6 +172,23 @@ def test_batch_codec_counts(orc, n):
         assert np.array_equal(got[:, :count], v) and not got[:, count:].any()
 
 
+@pytest.mark.parametrize("shift,stride", [(0, 4098), (0, 8192), (4096, 4096), (-4096, 4096), (5, 4097)])
+def test_batch_decode_over_its_plaintexts(orc, shift, stride):
+    """Slots that overlap other plaintexts than their own: several waves of transforms."""
+    n, batch = 4096, 800
+    t = orc.plain_modulus_batching(n, 20)
+    ctx = tb_capi.Context(BFV, n, orc.coeff_modulus_create(n, [40, 40]), t)
+    v = np.random.default_rng(stride).integers(0, t, (batch, n), dtype=np.uint64)
+    plain = _empty(batch, n)
+    ctx("batch_encode", _dev(v), 0, n, plain, batch, None)
+    buf = _empty((batch + 2) * max(n, stride) + abs(shift))
+    base = max(0, -shift)
+    buf[base:base + batch * n] = plain.view(-1)
+    ctx("batch_decode", buf[base:], buf[base + shift:], stride, batch, None)
+    got = _host(buf[base + shift:base + shift + batch * stride]).reshape(batch, stride)[:, :n]
+    assert np.array_equal(got, v)
+
+
 @pytest.mark.parametrize("size,pad", [(2, 0), (2, 1), (3, 0), (1, 3)])   # odd strides: 8-byte accesses
 def test_dyadic_accumulate_strides(orc, size, pad):
     n, L = 256, 2

@@ -118,3 +118,25 @@ def test_tables_of_a_context_are_on_the_device_when_it_is_returned(host, context
         assert kinds(records, "launch")
         assert not kinds(records, "race"), kinds(records, "race")
         """)
+
+
+@pytest.mark.parametrize("batch,shift,stride", [(3, 0, 4098), (3, 0, 8192), (2, 4096, 4096), (3, -4096, 4096),
+                                                (5, 8, 4096), (3, 0, 4096), (3, 0, 0), (3, 3 * 4096, 4100)])
+def test_batch_decode_reads_no_plaintext_that_it_may_have_written(host, batch, shift, stride):
+    """Slots over the plaintexts: the transforms of one launch run in any order, so unless
+    every plaintext is replaced by its own slots, they read a copy."""
+    host(f"""
+        n, batch, shift, stride = 4096, {batch}, {shift}, {stride}
+        c = context(SCHEME_BFV, n, 36, 36, 37)
+        base = words((2 * batch + 4) * 8192) + 8 * n
+        plain, slots = base, base + 8 * shift
+        records = calls(lambda: c("batch_decode", plain, slots, stride, batch, STREAM))
+        (stream, blocks, threads, src, dst, name), = [r for r in kinds(records, "launch") if "BatchDecodeOp" in r[5]]
+        s = stride or n
+        assert dst == slots
+        reads, writes = (src, src + 8 * batch * n), (dst, dst + 8 * ((batch - 1) * s + n))
+        disjoint = reads[1] <= writes[0] or writes[1] <= reads[0]
+        assert disjoint or (src == dst and s == n), (reads, writes)
+        copies = kinds(records, "copy")
+        assert src == plain or copies == [(STREAM, src, plain, 8 * batch * n)]
+        """)
