@@ -661,7 +661,12 @@ static int compose_level(Context &c, int L, const uint64_t *plain, double scale,
     uint64_t *tmp = nullptr;
     cudaError_t e = cudaMallocAsync(&tmp, 8ull * B * L * c.n, s);
     if (e != cudaSuccess) return status_from(e);
-    r = ntt_inverse(c, plain, tmp, B, 0, L, false, s);
+    // the transform loads pairs of words; a plaintext that starts inside a pair is copied first
+    if (reinterpret_cast<uintptr_t>(plain) & 15) {
+        r = status_from(cudaMemcpyAsync(tmp, plain, 8ull * B * L * c.n, cudaMemcpyDeviceToDevice, s));
+        plain = tmp;
+    }
+    if (r == TB_OK) r = ntt_inverse(c, plain, tmp, B, 0, L, false, s);
     if (r == TB_OK) {
         TraceScope ts("ckks_decode", s);
         launch_compose<MAX_COMPOSE_LT>(L, tmp, out, ostride, c, consts, 1.0 / scale, B, s);

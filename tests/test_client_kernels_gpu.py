@@ -120,6 +120,22 @@ def test_ckks_decode_limb_counts(orc, limbs):
     assert np.abs(got[:, 0] + 1j * got[:, 1] - exp).max() < 2.0 ** -25
 
 
+def test_ckks_decode_of_an_unaligned_plaintext(orc):
+    """A plaintext that starts in the middle of a 16-byte pair decodes like an aligned one."""
+    n, L, B = 4096, 2, 3
+    moduli = orc.coeff_modulus_create(n, [40, 40, 41])
+    ctx = tb_capi.Context(CKKS, n, moduli)
+    plain = _dev(_residues(np.random.default_rng(3), (B,), moduli[:L], n))
+    buf = _empty(B * L * n + 1)
+    buf[1:] = plain.view(-1)
+    assert buf[1:].data_ptr() % 16 == 8
+    for name in ("ckks_decode", "ckks_decode_polynomial"):
+        a, b = (torch.empty((B, n), dtype=torch.float64, device="cuda") for _ in range(2))
+        ctx(name, L, plain, 2.0 ** 40, a, 0, B, None)
+        ctx(name, L, buf[1:], 2.0 ** 40, b, 0, B, None)
+        assert torch.equal(a, b), name
+
+
 @pytest.mark.parametrize("scheme", [BFV, BGV, CKKS])
 def test_phase_of_larger_ciphertexts(orc, scheme):
     """Decryption of sizes 2 .. 4 with strides: c_0 + c_1 s + c_2 s^2 + ..."""

@@ -140,3 +140,20 @@ def test_batch_decode_reads_no_plaintext_that_it_may_have_written(host, batch, s
         copies = kinds(records, "copy")
         assert src == plain or copies == [(STREAM, src, plain, 8 * batch * n)]
         """)
+
+
+@pytest.mark.parametrize("call", ["ckks_decode", "ckks_decode_polynomial"])
+@pytest.mark.parametrize("offset", [0, 8])
+def test_ckks_decode_transforms_aligned_words(host, call, offset):
+    """The transforms load pairs of words at once; a plaintext that starts in the middle of
+    a pair is copied first."""
+    host(f"""
+        c = context(SCHEME_CKKS, 4096, 40, 40, 41)
+        plain = words(3 * 4096) + {offset}
+        records = calls(lambda: c("{call}", 2, plain, 2.0 ** 30, words(4096), 0, 1, STREAM))
+        (stream, blocks, threads, src, dst, name), = [r for r in kinds(records, "launch") if "PlainNttOp" in r[5]]
+        assert src % 16 == 0 and dst % 16 == 0, (src, dst)
+        copies = kinds(records, "copy")
+        assert src == plain or copies == [(STREAM, src, plain, 8 * 2 * 4096)]
+        assert (src == plain) == ({offset} == 0)
+        """)
