@@ -169,9 +169,12 @@ int context_create(int scheme, uint64_t n, const uint64_t *moduli, int count, ui
         for (auto p : extra) c->table_moduli.push_back(p);
     }
     const size_t nm = c->table_moduli.size();
-    // per modulus: forward and inverse twiddles, and both again in the order of the radix-8
-    // passes (fp64mod.cuh), 2 N further on
-    std::vector<ulonglong2> all(4 * nm * n);
+    // per modulus: forward and inverse twiddles, and, 2 N further on, both again in the order
+    // of the radix-8 passes (fp64mod.cuh), which the transforms of whole limbs in one CTA
+    // read (up to 2^14 coefficients)
+    const bool ordered = c->logn <= MAX_LOGB;
+    const size_t per = (ordered ? 4 : 2) * n;
+    std::vector<ulonglong2> all(per * nm);
     c->h_mods.resize(nm);
     for (size_t i = 0; i < nm; i++) {
         std::vector<ulonglong2> f, v;
@@ -179,9 +182,10 @@ int context_create(int scheme, uint64_t n, const uint64_t *moduli, int count, ui
             delete c;
             return set_error(TB_ERR_INVALID_ARGUMENT, "modulus has no primitive 2N-th root of unity");
         }
-        ulonglong2 *t = &all[4 * i * n];
+        ulonglong2 *t = &all[per * i];
         std::memcpy(t, f.data(), n * sizeof(ulonglong2));
         std::memcpy(t + n, v.data(), n * sizeof(ulonglong2));
+        if (!ordered) continue;
         t[2 * n] = f[0];
         t[3 * n] = v[0];
         for (uint32_t k = 1; k < n; k++) {
@@ -195,8 +199,8 @@ int context_create(int scheme, uint64_t n, const uint64_t *moduli, int count, ui
         return status_from(e);
     }
     for (size_t i = 0; i < nm; i++) {
-        c->h_mods[i].roots = c->d_tables + 4 * i * n;
-        c->h_mods[i].inv_roots = c->d_tables + (4 * i + 1) * n;
+        c->h_mods[i].roots = c->d_tables + per * i;
+        c->h_mods[i].inv_roots = c->h_mods[i].roots + n;
     }
     e = build_fp_tables(*c);
     if (e == cudaSuccess) e = to_device(c->h_mods.data(), nm, &c->d_mods);

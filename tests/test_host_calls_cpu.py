@@ -157,3 +157,14 @@ def test_ckks_decode_transforms_aligned_words(host, call, offset):
         assert src == plain or copies == [(STREAM, src, plain, 8 * 2 * 4096)]
         assert (src == plain) == ({offset} == 0)
         """)
+
+
+@pytest.mark.parametrize("n,tables", [(8192, 4), (16384, 4), (32768, 2), (65536, 2)])
+def test_twiddle_memory(host, n, tables):
+    """Twiddles in natural order, forward and inverse, and again in the order of the radix-8
+    passes where one CTA transforms a whole limb (up to 2^14 coefficients) and reads that."""
+    host(f"""
+        moduli = primes({n}, 60, 60, 60)
+        records = calls(lambda: tb_capi.Context(SCHEME_RAW, {n}, moduli, 0))
+        assert max(b for _, b in kinds(records, "malloc")) == 16 * {n} * {tables} * len(moduli)
+        """)
