@@ -397,7 +397,7 @@ int tb_negate(tb_context *ctx, int L, int size, const uint64_t *a, uint64_t a_st
 /* NTT launch variant for one direction and log2 block size (12..14 have variants 0 to
    5: 0, 1 and 2 the default thread count, half and a quarter of it, each thread taking
    correspondingly more radix-8 groups per pass, fewer threads letting several limbs
-   share an SM (at variant 0 a launch of many 2^12 or 2^13 limbs takes variant 1's count);
+   share an SM;
    3, 4 and 5 transform a whole limb on a cluster of two CTAs holding half
    of it each, with the thread counts of 0, 1 and 2 for the half block, and launch the
    sub-blocks of longer limbs as 0, 1 and 2). */
@@ -405,9 +405,10 @@ int tb_ntt_set_variant(int forward, int log_block, int variant);
 int tb_ntt_get_variant(int forward, int log_block, int *variant);
 /* On (the default): a launch of whole 2^12..2^14 limbs with at most half as many limbs
    as the device has SMs takes the two-CTA form of its variant (0 -> 3, 1 -> 4, 2 -> 5),
-   so small batches (one ciphertext per call) occupy twice as many SMs, and a launch of at
-   most a quarter as many whole 2^12..2^15 limbs runs each on a cluster of eight CTAs; off:
-   every launch takes the set variant. */
+   so small batches (one ciphertext per call) occupy twice as many SMs, a launch of at
+   most a quarter as many whole 2^12..2^15 limbs runs each on a cluster of eight CTAs, and
+   a launch of at least six 2^12 or three 2^13 limbs per SM takes variant 1's thread count
+   at variant 0; off: every launch takes the set variant. */
 int tb_ntt_set_small_launch_pairs(int on);
 /* Times every variant of the context's transform size on `polys` scratch limbs (0 =
    256) with CUDA events on `stream` and keeps the fastest per direction. */

@@ -145,7 +145,9 @@ static_assert(!fwd_subtracts(64, 16), "no subtraction in the wide form");
 // CTA per limb: no subtraction at all and the estimated quotient, ct_butterfly_wide;
 // from inputs below B the outputs stay below B + 4 q log2 N, below 2^61 + 56 q < 2^63.2
 // for inputs below 2^61 at N <= 16384). The Op takes those outputs at its store. The
-// CTA-pair and cluster forms always run the Harvey stages (outputs below 4q).
+// CTA-pair, eight-CTA and cluster forms always run the Harvey stages: outputs below 4q from
+// inputs below 4q. Where an Op's wide form loads unreduced words below B > 4q, theirs stay
+// below B: a stage takes 2q from such an x before it adds less than 2q.
 constexpr int SLACK_M = 16;
 constexpr int SLACK_WIDE = 64;
 template <class Ctx, class = void>
@@ -1281,7 +1283,7 @@ inline cudaError_t launch_inv(const Op &op, unsigned blocks, int logn, int scale
 int ntt_variant(bool fwd, int logb);
 // Streaming multiprocessors of the current device (cached per device).
 int sm_count();
-// Whether launches of fewer limbs than SMs take the two-CTA form (tb_ntt_set_small_launch_pairs).
+// Whether launches take forms by their number of limbs (tb_ntt_set_small_launch_pairs).
 bool small_launch_pairs();
 
 // Whole limbs of 2^(LOGB+1) coefficients, one CTA pair each (forward from stage 0,
@@ -1452,12 +1454,15 @@ inline int small_launch_variant(int v, unsigned blocks) {
 
 // A launch of many limbs of 2^12 or 2^13 coefficients with half the threads per limb, two
 // groups a thread and pass: twice as many limbs share an SM (2^13: 2 of 512 threads, 2^12:
-// 4 of 256), and one limb's loads, barriers and stores overlap another's arithmetic. 256
-// polynomials x 6 limbs at N = 8192: forward 124 -> 95 us, inverse 121 -> 105 us. Below one
-// and a half waves of them the longer limbs cost more than they overlap (66 limbs: 58 ->
-// 62 us, 396 limbs: 33 -> 38 us, 528 limbs: 45 -> 37 us).
+// 4 of 256), and one limb's loads, barriers and stores overlap another's arithmetic. Plain
+// transforms at N = 8192: 1536 limbs forward 117 -> 86 us, inverse 121 -> 100 us, 528 limbs
+// 49 -> 39 and 48 -> 43 us. The line, three (six) limbs per SM, is where the fused transforms
+// with epilogues stop losing: below it their fewer, longer CTAs leave SMs idle (BGV chains of
+// 16 pairs, 96 - 128 limbs a launch: mod-down 50 -> 62 us; of 20 - 24 pairs: special-prime
+// inverse 52 -> 78 us, mod-down 69 -> 71), although the mod-up and plain transforms gain there
+// too (16 pairs: 58 -> 50 us; 396 limbs: 39 -> 31). Off with the rule for small launches.
 inline int large_launch_variant(int v, int logb, unsigned blocks) {
-    if (v != 0) return v;
+    if (v != 0 || !small_launch_pairs()) return v;
     const unsigned sms = (unsigned)sm_count();
     return (logb == 13 && blocks >= 3 * sms) || (logb == 12 && blocks >= 6 * sms) ? 1 : 0;
 }

@@ -168,3 +168,31 @@ def test_twiddle_memory(host, n, tables):
         records = calls(lambda: tb_capi.Context(SCHEME_RAW, {n}, moduli, 0))
         assert max(b for _, b in kinds(records, "malloc")) == 16 * {n} * {tables} * len(moduli)
         """)
+
+
+@pytest.mark.parametrize("logn,limbs", [(12, 37), (12, 6 * 148), (13, 37), (13, 3 * 148), (14, 74)])
+@pytest.mark.parametrize("forward", [0, 1])
+def test_size_rules_are_off_with_the_switch(host, logn, limbs, forward):
+    """Launches of few and of many limbs take the set variant with the small-launch rules
+    off, and forms of their own with them on."""
+    host(f"""
+        logn, limbs, forward = {logn}, {limbs}, {forward}
+        n = 1 << logn
+        c = context(SCHEME_RAW, n, 40)
+        x = words(limbs * n)
+
+        def shape():
+            records = calls(lambda: c("ntt_forward" if forward else "ntt_inverse", x, x, limbs, 0, 1, 0, STREAM))
+            (stream, blocks, threads, src, dst, name), = kinds(records, "launch")
+            return blocks, threads
+
+        own = shape()
+        lib.tb_ntt_set_small_launch_pairs(0)
+        for v in (0, 1, 2):
+            tb_capi.check(lib.tb_ntt_set_variant(forward, logn, v))
+            assert shape() == (limbs, min(1024, n // 8) >> v), v
+        tb_capi.check(lib.tb_ntt_set_variant(forward, logn, 0))
+        assert own != shape()
+        lib.tb_ntt_set_small_launch_pairs(1)
+        assert own == shape()
+        """)
