@@ -1115,6 +1115,10 @@ def main():
     if args.impl == "reference":
         if rank != 0:
             return
+        if not os.path.exists(os.path.join(ROOT, "oracle", "_ref", "libtroyref.so")):
+            print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/libtroyref.so is not built (it is "
+                              "compiled from the reference's sources, which are not on this machine)"}))
+            return
         workers = cores
         vals = []
         for i in range(args.warmup + args.steps):

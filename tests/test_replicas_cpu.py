@@ -1,6 +1,7 @@
-"""The multi-GPU path of bench.py (replicas, one process per GPU) on CPU: two gloo
-ranks with different timings combine to the slowest rank's times and the whole-job
-rate counts both ranks' work; with one rank nothing is exchanged."""
+"""The host-side parts of bench.py on CPU. Its multi-GPU path (replicas, one process per
+GPU): two gloo ranks with different timings combine to the slowest rank's times and the
+whole-job rate counts both ranks' work; with one rank nothing is exchanged. The reference
+arm without its library."""
 import os
 import socket
 import sys
@@ -75,3 +76,15 @@ def test_sub_batches_keep_every_pairs_rotation_step():
         assert got == whole
         rows = ckks_step.row_groups(pairs, count, steps)
         assert len(rows) == pairs and {g: rows.count(g) for g in set(rows)} == whole
+
+
+def test_reference_arm_without_its_library(monkeypatch, capsys, tmp_path):
+    """One JSON line that says why, and a normal exit."""
+    import json
+    sys.path.insert(0, ROOT)
+    import bench
+    monkeypatch.setattr(bench, "ROOT", str(tmp_path))
+    monkeypatch.setattr(sys, "argv", ["bench.py", "--impl", "reference", "--steps", "1", "--warmup", "0"])
+    bench.main()
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and "libtroyref.so" in line["unavailable"]
