@@ -33,41 +33,115 @@ def _residues(rng, lead, moduli, n):
     return np.stack([rng.integers(0, q, tuple(lead) + (n,), dtype=np.uint64) for q in moduli], -2)
 
 
-@pytest.mark.parametrize("scheme", [BFV, BGV, CKKS])
-@pytest.mark.parametrize("count", [1, 3, 40])   # 40: several refills of the stream per CTA
-def test_batched_encryption_words(orc, scheme, count):
-    """Every encryption of a seeded batch has the oracle's words (each starts the seed's
-    stream anew), and decrypts to its plaintext."""
+def _with_plain(O, scheme, ct, plain):
+    """ct, an encryption of zero from the oracle, plus the plaintext (as Encryptor does)."""
+    ct = ct.copy()
+    data = O.moduli[:ct.shape[1]]
+    if scheme == BFV:
+        ct[0] = O._multiply_add_plain_scaling_variant(data, ct[0], plain)
+    else:
+        ct[0] = np.stack([((ct[0, l].astype(object) + (plain[l] if scheme == CKKS else plain).astype(object)) % q)
+                          for l, q in enumerate(data)]).astype(np.uint64)
+    return ct
+
+
+def _client(orc, scheme, seedp):
+    """Context of three primes (two data primes), secret and public key."""
     n = 4096
     moduli = orc.coeff_modulus_create(n, [36, 36, 40])
     t = orc.plain_modulus_batching(n, 20) if scheme != CKKS else 0
-    K, L = 3, 2
     ctx = tb_capi.Context(scheme, n, moduli, t)
+    sk, pk = _empty(3, n), _empty(2, 3, n)
+    ctx("keygen_secret", seedp, sk, None)
+    ctx("keygen_public", seedp, sk, pk, None)
+    return n, moduli, t, ctx, sk, pk
+
+
+def _plains(rng, scheme, count, moduli, t, n):
+    return _residues(rng, (count,), moduli, n) if scheme == CKKS else rng.integers(0, t, (count, n), dtype=np.uint64)
+
+
+@pytest.mark.parametrize("scheme", [BFV, BGV, CKKS])
+@pytest.mark.parametrize("count", [1, 3, 40])   # 40: several refills of the stream per CTA
+def test_batched_encryption_words(orc, scheme, count):
+    """Every encryption of a seeded batch has the oracle's words for its own plaintext (each
+    starts the seed's stream anew), asymmetric and symmetric, with padded strides too, and
+    decrypts to its plaintext."""
+    n, moduli, t, ctx, sk, pk = _client(orc, scheme, SEEDP)
     O = OracleSession(scheme, n, moduli, t, SEED)
-    sk, pk = _empty(K, n), _empty(2, K, n)
-    ctx("keygen_secret", SEEDP, sk, None)
-    ctx("keygen_public", SEEDP, sk, pk, None)
-    rng = np.random.default_rng(5)
-    if scheme == CKKS:
-        plain = _residues(rng, (), moduli[:L], n)
-    else:
-        plain = rng.integers(0, t, n, dtype=np.uint64)
-    exp = np.asarray(O.encrypt_plain(plain)).reshape(2, L, n)
-    out = _empty(count, 2, L, n)
-    plains = _dev(np.broadcast_to(plain, (count,) + plain.shape))
-    ctx("encrypt", SEEDP, pk, L, plains, plain.size, n, out, 0, count, None)
-    got = _host(out)
-    for i in range(count):
-        assert np.array_equal(got[i], exp), i
-    sym = _empty(count, 2, L, n)
-    ctx("encrypt_symmetric", SEEDP, sk, L, plains, plain.size, n, sym, 0, count, None)
-    gs = _host(sym)
-    assert all(np.array_equal(gs[i], gs[0]) for i in range(count))
-    if scheme != CKKS:
-        for ct in (out, sym):
+    L, ckks = 2, scheme == CKKS
+    plain = _plains(np.random.default_rng(5), scheme, count, moduli[:L], t, n)
+    zero = np.zeros((L, n) if ckks else n, np.uint64)
+    zeros = {"encrypt": (np.asarray(O.encrypt_plain(zero)).reshape(2, L, n), pk),
+             "encrypt_symmetric": (O.encrypt_zero_symmetric(moduli[:L], ckks), sk)}
+    for name, (z, key) in zeros.items():
+        for pad in (0, 2):
+            padded = np.zeros((count, zero.size + pad), np.uint64)
+            padded[:, :zero.size] = plain.reshape(count, -1)
+            out = _empty(count, 2 * L * n + pad)
+            ctx(name, SEEDP, key, L, _dev(padded), zero.size + pad, n, out, 2 * L * n + pad, count, None)
+            got = np.ascontiguousarray(_host(out)[:, :2 * L * n]).reshape(count, 2, L, n)
+            for i in range(count):
+                assert np.array_equal(got[i], _with_plain(O, scheme, z, plain[i])), (name, pad, i)
+        if not ckks:
             dec = _empty(count, n)
-            ctx("decrypt", sk, L, 2, ct, 0, dec, 0, 1, count, None)
-            assert np.array_equal(_host(dec), _host(plains))
+            ctx("decrypt", sk, L, 2, _dev(got), 0, dec, 0, 1, count, None)
+            assert np.array_equal(_host(dec), plain), name
+    if not ckks and count == 1:   # the oracle's own encryption of a plaintext
+        assert np.array_equal(_with_plain(O, scheme, zeros["encrypt"][0], plain[0]),
+                              np.asarray(O.encrypt_plain(plain[0])).reshape(2, L, n))
+
+
+@pytest.mark.parametrize("scheme", [BFV, BGV, CKKS])
+def test_every_encryption_of_a_batch_has_samples_of_its_own(orc, scheme):
+    """Without a seed each ciphertext draws its own u, e_0 and e_1. The public key (1000, 0)
+    and no dropped prime make them readable: c_0 = 1000 u + e_0 (t e_0 for BGV), c_1 = e_1."""
+    n, moduli, t, ctx, sk, _ = _client(orc, scheme, None)
+    K, count = 3, 6
+    factor = t if scheme == BGV else 1
+    scale = 1000 * factor   # above 2 x 21 factor, the binomial samples' range
+    pk = np.zeros((2, K, n), np.uint64)
+    pk[0] = scale
+    out = _empty(count, 2, K, n)
+    ctx("encrypt", None, _dev(pk), K, None, 0, 0, out, 0, count, None)
+    seen = {"u": set(), "e0": set(), "e1": set()}
+    for ct in _host(out):
+        if scheme == CKKS:
+            ct = np.stack([orc.ntt_inverse_rns(12, moduli, p) for p in ct])
+        q = np.array(moduli, np.int64)[None, :, None]
+        c = ct.astype(np.int64)
+        c = np.where(c > q // 2, c - q, c)
+        assert (c == c[:, :1]).all()   # the same integers modulo every prime
+        u = np.rint(c[0, 0] / scale).astype(np.int64)
+        e0, e1 = c[0, 0] - scale * u, c[1, 0]
+        assert not (e0 % factor).any() and not (e1 % factor).any()
+        for name, v, top in (("u", u, 1), ("e0", e0 // factor, 21), ("e1", e1 // factor, 21)):
+            assert abs(v).max() <= top and len(set(v.tolist())) > 2, name
+            seen[name].add(v.tobytes())
+    assert all(len(v) == count for v in seen.values())
+
+
+@pytest.mark.parametrize("scheme", [BFV, BGV, CKKS])
+def test_unseeded_batches_decrypt(orc, scheme):
+    """Batches without a seed: no two ciphertexts share c_1, and each decrypts to its own
+    plaintext (CKKS: up to the dropped prime's rounding, (n + 1) / 2 and the noise)."""
+    n, moduli, t, ctx, sk, pk = _client(orc, scheme, None)
+    L, count = 2, 5
+    plain = _plains(np.random.default_rng(7), scheme, count, moduli[:L], t, n)
+    for name, key in (("encrypt", pk), ("encrypt_symmetric", sk)):
+        out = _empty(count, 2, L, n)
+        ctx(name, None, key, L, _dev(plain), plain[0].size, n, out, 0, count, None)
+        assert len({c.tobytes() for c in _host(out)[:, 1]}) == count, name
+        dec = _empty(count, L, n) if scheme == CKKS else _empty(count, n)
+        ctx("decrypt", sk, L, 2, out, 0, dec, 0, 1, count, None)
+        got = _host(dec)
+        if scheme != CKKS:
+            assert np.array_equal(got, plain), name
+            continue
+        for b in range(count):
+            for l, q in enumerate(moduli[:L]):
+                noise = orc.ntt_inverse(12, q, (got[b, l] + np.uint64(q) - plain[b, l]) % np.uint64(q)).astype(np.int64)
+                assert abs(np.where(noise > q // 2, noise - q, noise)).max() < n, (name, b, l)
 
 
 @pytest.mark.parametrize("logn", [6, 12, 13, 14, 15, 16])

@@ -300,3 +300,39 @@ def test_wide_form_takes_unreduced_inputs(orc):
     got = _host(out)
     for p in range(3):
         assert np.array_equal(got[p], orc.rns_op("div_round_last_ntt", n, data, 0, x[p], L)[: L - 1]), p
+
+
+@pytest.mark.parametrize("scheme", [BFV, BGV, CKKS])
+@pytest.mark.parametrize("L", [1, 8, 9, 17])
+def test_keyswitch_fp64_sums(orc, scheme, L):
+    """The inner products of moduli below 2^50 are exact FP64 sums, reduced every eight
+    digits: the largest primes below 2^50, up to 17 digits, and constant target polynomials
+    q_j - 1, so that every digit is known: modulo the larger primes it is just below the
+    modulus. Key words by coefficient: q - 1 (the largest products), the ones that make
+    every term the residue (q - 1) / 2 or (q + 1) / 2 (the largest sums, of either sign),
+    and random ones near q."""
+    n, logn = 4096, 12
+    moduli = orc.coeff_modulus_create(n, [50] * 18)
+    assert all((1 << 49) < q < (1 << 50) for q in moduli) and moduli[-1] == max(moduli)
+    t = 0 if scheme == CKKS else orc.plain_modulus_batching(n, 20)
+    ctx = tb_capi.Context(scheme, n, moduli, t)
+    K = len(moduli)
+    rng = np.random.default_rng(50)
+    key = np.empty((K - 1, 2, K, n), np.uint64)
+    for i, q in enumerate(moduli):
+        near = rng.integers(q - (q >> 20), q, (K - 1, 2, n), dtype=np.uint64)
+        for j in range(K - 1):
+            inv = pow((moduli[j] - 1) % q, -1, q)
+            words = np.array([q - 1, (q - 1) // 2 * inv % q, (q + 1) // 2 * inv % q, 0], np.uint64)
+            key[j, :, i] = np.resize(words, n)
+            key[j, :, i, 3::4] = near[j, :, 3::4]
+    data = moduli[:L]
+    target = np.zeros((1, L, n), np.uint64)
+    for j, q in enumerate(data):
+        target[0, j, slice(None) if scheme == CKKS else 0] = q - 1   # NTT form: constant words
+    ct = _rand(rng, data, n, (1, 2))
+    dct = _dev(ct)
+    ctx("keyswitch", L, _dev(target), 0, dct, 0, _dev(key), 1, None)
+    exp = orc.keyswitch(scheme, logn, data + [moduli[-1]], t, target[0], ct[0], _key_sub(key, L))
+    assert np.array_equal(_host(dct)[0], exp)
+    ctx.close()

@@ -2,8 +2,10 @@
 oracle, word for word: primes at the edges of the form (the largest below 2^48, which run
 without reductions, the largest below 2^49 and 2^50, which reduce at every pass, the first
 one above 2^50, in integer form, and small ones), extreme inputs (all q - 1, alternating,
-up to 4 q - 1 where the transforms take lazy words), and launches of one limb (CTA pairs),
-of a few and of enough limbs for every launch rule."""
+up to 4 q - 1 where the transforms take lazy words), and launches on both sides of every
+size rule, which count limbs against the device's SMs: up to a quarter of them clusters of
+eight CTAs, up to half CTA pairs, then one CTA a limb (2^15: CTA pairs), and from three
+(2^13) or six (2^12) limbs an SM on half the threads."""
 import numpy as np
 import pytest
 
@@ -30,6 +32,13 @@ def _rows(n, q, top, seed):
     return rows
 
 
+def _counts(logn):
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    many = {12: 6 * sms, 13: 3 * sms}.get(logn)
+    return sorted({1, 4, sms // 4, sms // 4 + 1, sms // 2, sms // 2 + 1, sms + 12,
+                   *((many - 1, many, many + 12) if many else (460,))})
+
+
 @pytest.mark.parametrize("logn", [12, 13, 14, 15])
 @pytest.mark.parametrize("kind", ["20", "40", "48", "49", "50", "above50"])
 def test_fp64_transforms(orc, logn, kind):
@@ -41,7 +50,7 @@ def test_fp64_transforms(orc, logn, kind):
         fwd = np.stack([orc.ntt_forward(logn, q, r) for r in rows])
         lazy = rows % np.uint64(2 * q)   # the inverse takes words below 2 q
         inv = np.stack([orc.ntt_inverse(logn, q, r) for r in lazy])
-        for polys in (1, 4, 160, 900 if logn == 12 else 460):
+        for polys in _counts(logn):
             x = _dev(np.ascontiguousarray(np.resize(rows, (polys, n))))
             out = torch.empty_like(x)
             ctx("ntt_forward", x, out, polys, 0, 1, 0, None)
