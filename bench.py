@@ -15,16 +15,16 @@ prime (the arithmetic performed is the same as on encrypted data).
 
 * ``value``: ops/s with inputs resident in HBM (CUDA events on the launch stream,
   max over ranks). Inputs (2 x 128 MB) exceed the 126 MB L2 between steps. Each
-  step's 64 pairs run as S concurrent sub-batches, one stream each (default 4), the
+  step's 64 pairs run as S concurrent sub-batches, one stream each (default 2), the
   whole fork/join captured once as a CUDA graph and replayed per step (--no-graph:
   eager launches).
 * ``e2e``: the same metric through the C ABI with host buffers: every step copies
-  both operand batches from pinned host memory and reads the results back, as 4
+  both operand batches from pinned host memory and reads the results back, as 2
   sub-batches whose copies run on one stream per direction, overlapping the
-  neighbouring sub-batches' arithmetic (two device buffer sets, ordered by events).
+  neighbouring sub-batches' arithmetic (three device buffer sets, ordered by events).
 * ``roofline``: the dominant kernel from the library's per-launch event trace of the
   same steps run as one batch on one stream, against the measured HBM copy peak and
-  (``roofline.int``) the measured integer ceiling of the transforms.
+  (``roofline.arith``) the measured arithmetic ceiling of the transforms.
 * ``cpu_baseline``: the reference's own CPU implementation (compiled under
   oracle/_ref) on a bounded sample of the same workload, one process per core.
 * ``plain_per_op``: the same chain driven one pair per call (batch 1), as the
@@ -34,7 +34,7 @@ prime (the arithmetic performed is the same as on encrypted data).
   per call, in a child process; ``batched_over_reference_gpu_per_op`` compares.
 * ``ntt_sweep``: the raw NTT / dyadic / inverse NTT workload (256 x 8 limbs, N =
   4096 .. 32768) with GB/s and fraction of the measured copy peak per kernel, and of
-  the integer ceiling per transform.
+  the FP64 ceiling per transform.
 * ``uneven_batch``: 512 BFV/BGV ciphertexts of degrees 4096 / 8192 / 16384 through
   multiply, relinearize and rotate_rows as one captured CUDA graph, beside the
   one-ciphertext-per-call path.
@@ -433,8 +433,11 @@ def run_b200(args, rank, world):
             "h2d_seeded": (hA0.numel() + hB0.numel() + hSA.numel() + hSB.numel()) * 8,
             "ms": ms, "e2e_ms": e2e_ms, "per_op_ms": per_op_ms, "per_op_pairs": per_op_pairs, "trace": trace, "launches": launches, "clocks": clk,
             "h2d": (A.numel() + B.numel()) * 8, "d2h": O.numel() * 8, "L": L, "K": K, "e2e_chunks": CH,
-            "int_ceiling": int_ceiling(lib, moduli[0]), "int_ceiling_slack": int_ceiling(lib, moduli[0], kind="slack"),
-            "int_ceiling_wide": int_ceiling(lib, moduli[0], kind="wide"), "mul64": mul64_rates(lib),
+            "butterfly_rates": {"harvey": butterfly_rate(lib, moduli[0]),
+                                "slack": butterfly_rate(lib, moduli[0], "slack"),
+                                "wide": butterfly_rate(lib, moduli[0], "wide"),
+                                "fp64": butterfly_rate(lib, min(moduli), "fp64")},
+            "mul64": mul64_rates(lib),
             "butterfly_mix": butterfly_mix(moduli, L, N.bit_length() - 1), "sub": SUB}
 
 
@@ -443,10 +446,9 @@ def run_ntt_sweep(batch=256, reps=10):
     N in {4096, ..., 32768}: forward NTT, dyadic product of pairs, inverse NTT.
     Algorithmic bytes: 16 N B L per transform (read + write), 24 N B L per dyadic
     product; GB/s and the fraction of the measured copy peak per kernel, and for the
-    transforms the fraction of the integer ceiling ((N/2) log2 N butterflies per limb
-    over tb_measure_butterfly_rate; the forward transform (full outputs, deferred
-    reductions) over that rate and tb_measure_slack_butterfly_rate weighted by the
-    shares of its stages that run each butterfly)."""
+    transforms the fraction of the arithmetic ceiling of the form they run, exact FP64
+    for these moduli: (N/2) log2 N butterflies per limb over
+    tb_measure_fp64_butterfly_rate."""
     import torch
     import tb_capi
 
@@ -465,11 +467,7 @@ def run_ntt_sweep(batch=256, reps=10):
         tb_capi.check(lib.tb_coeff_modulus_create(ctypes.c_uint64(n), arr, 8, mods))
         moduli = [int(m) for m in mods]
         if ceiling is None:
-            ceiling = int_ceiling(lib, moduli[0])
-            ceiling_slack = int_ceiling(lib, moduli[0], kind="slack")
-        # forward: stages above 2^14 run separately (Harvey), the 2^14 blocks defer
-        sh = (min(logn, 14) - fwd_subtracting_stages(min(logn, 14))) / logn
-        ceilings = {"ntt_forward": 1.0 / (sh / ceiling_slack + (1.0 - sh) / ceiling), "ntt_inverse": ceiling}
+            ceiling = butterfly_rate(lib, moduli[0], "fp64")
         ctx = tb_capi.Context(tb_capi.SCHEME_RAW, n, moduli)
         x = _rand_residues(torch, (batch, 8, n), moduli, gen)
         y = _rand_residues(torch, (batch, 8, n), moduli, gen)
@@ -503,9 +501,9 @@ def run_ntt_sweep(batch=256, reps=10):
                                  ("ntt_inverse", ms_i, 16 * words)):
             gbs = bytes_ / (ms * 1e-3) / 1e9
             row[name] = {"ms": round(ms, 4), "GBps": round(gbs, 1), "frac_of_measured_hbm": round(gbs / peak, 4)}
-            if name != "dyadic":   # against the integer ceiling: (N/2) log2 N butterflies per limb
+            if name != "dyadic":   # (N/2) log2 N butterflies per limb
                 rate = batch * 8 * (n // 2) * logn / (ms * 1e-3)
-                row[name]["frac_of_int_ceiling"] = round(rate / ceilings[name], 4)
+                row[name]["frac_of_fp64_ceiling"] = round(rate / ceiling, 4)
         row["variants"] = {"forward": vf.value, "inverse": vi.value}
         out[f"N={n}"] = row
         for fwd, v in zip((1, 0), saved):
@@ -513,8 +511,7 @@ def run_ntt_sweep(batch=256, reps=10):
         del x, y, z
         ctx.close()
     return {"workload": f"{batch} polynomials x 8 limbs (50-bit primes)",
-            "int_ceiling_gbutterflies_per_s": round(ceiling / 1e9, 2),
-            "int_ceiling_slack_gbutterflies_per_s": round(ceiling_slack / 1e9, 2), "results": out}
+            "fp64_ceiling_gbutterflies_per_s": round(ceiling / 1e9, 2), "results": out}
 
 
 UNEVEN_SHAPES = [(1, 4096, [36, 36, 37]), (3, 8192, [43, 43, 44, 44, 44]), (1, 16384, [48] * 9)]
@@ -806,30 +803,19 @@ def roofline(res, steps):
     bpl = alg[name] * steps / launches
     achieved = bpl / (per_launch_ms * 1e-3) / 1e9
     tr = measured_traffic().get(name)
-    # the transforms against the integer ceiling (butterflies per second)
+    # the transforms against the arithmetic ceiling (butterflies per second): the rates of
+    # the butterflies they run, weighted by the shares of each kind
     bfly = butterflies_per_step(res["L"])
-    ceil_std = res.get("int_ceiling")
-    ceilings = {}
-    if ceil_std:
-        ceilings = {k: ceil_std for k in bfly}
-        if res.get("int_ceiling_slack") and res.get("int_ceiling_wide"):
-            # the forward transforms run three kinds of butterfly: their ceiling is the
-            # three rates weighted by the kinds' shares of their butterflies
-            rates = {"harvey": ceil_std, "slack": res["int_ceiling_slack"], "wide": res["int_ceiling_wide"]}
-            for k, mix in res["butterfly_mix"].items():
-                ceilings[k] = 1.0 / sum(sh / rates[kind] for kind, sh in mix.items())
+    rates = res["butterfly_rates"]
+    ceilings = {k: 1.0 / sum(sh / rates[kind] for kind, sh in mix.items()) for k, mix in res["butterfly_mix"].items()}
     for k, row in table.items():
-        if k in bfly and k in ceilings:
-            rate = bfly[k] / (row["ms_per_step"] * 1e-3)
-            row["int_frac"] = round(rate / ceilings[k], 4)
-    ceil = ceilings.get(name)
+        if k in bfly:
+            row["arith_frac"] = round(bfly[k] / (row["ms_per_step"] * 1e-3) / ceilings[k], 4)
     # the roofline is stated against HBM (achieved / peak in GB/s); "limited_by" names the
-    # resource the kernel uses the larger fraction of: HBM bandwidth, or the integer
-    # ceiling of the transforms ("int" sub-object)
-    int_frac = None
-    if name in bfly and ceil:
-        int_frac = bfly[name] * steps / launches / (per_launch_ms * 1e-3) / ceil
-    limited_by = "int" if int_frac is not None and int_frac > achieved / peak else "hbm"
+    # resource the kernel uses the larger fraction of: HBM bandwidth, or the arithmetic
+    # ceiling of the transforms ("arith" sub-object)
+    rate = bfly[name] * steps / launches / (per_launch_ms * 1e-3) if name in bfly else None
+    limited_by = "arith" if rate and rate / ceilings[name] > achieved / peak else "hbm"
     out = {"kernel": name, "bound": "hbm", "limited_by": limited_by, "achieved": round(achieved, 1), "peak": peak,
            "unit": "GB/s",
            "frac": round(achieved / peak, 4),
@@ -842,32 +828,24 @@ def roofline(res, steps):
     if res.get("sub", 1) > 1:
         out["timing"] = (f"kernel times from the same {steps} steps run as one batch on one stream after the "
                          f"timed region (which runs {res['sub']} concurrent sub-batches)")
-    if name in bfly and ceil:
-        rate = bfly[name] * steps / launches / (per_launch_ms * 1e-3)
-        out["int"] = {"achieved": round(rate / 1e9, 2), "peak": round(ceil / 1e9, 2), "unit": "Gbutterfly/s",
-                      "frac": round(rate / ceil, 4), "butterflies_per_launch": round(bfly[name] * steps / launches),
-                      "peak_source": "measured here: tb_measure_butterfly_rate, operands in registers"}
-        m = res.get("mul64")
-        if m:
-            # the machine bound of an exact-quotient butterfly: its Shoup product is one
-            # high and two low 64-bit products (the wide form estimates its quotient from
-            # 32-bit products and may pass it)
-            bound = 1.0 / (1.0 / m["hi"] + 2.0 / m["lo"])
-            out["int"]["machine_bound"] = {
-                "mul_lo_per_s": round(m["lo"] / 1e9, 1), "mul_hi_per_s": round(m["hi"] / 1e9, 1), "unit": "G/s",
-                "butterflies_per_s": round(bound / 1e9, 2), "frac": round(rate / bound, 4),
-                "ceiling_frac": round(ceil / bound, 4),
-                "source": "tb_measure_mul64_rate: mul.lo.u64 / mul.hi.u64 in independent chains; "
-                          "bound = 1 / (1/hi + 2/lo) butterflies per second"}
-        if name in res.get("butterfly_mix", {}) and res.get("int_ceiling_wide"):
-            mix = res["butterfly_mix"][name]
-            out["int"]["peak_source"] = (
-                "measured here, operands in registers: tb_measure_butterfly_rate "
-                f"({ceil_std / 1e9:.2f} G/s), tb_measure_slack_butterfly_rate "
-                f"({res['int_ceiling_slack'] / 1e9:.2f} G/s) and tb_measure_wide_butterfly_rate "
-                f"({res['int_ceiling_wide'] / 1e9:.2f} G/s), weighted by the shares of the kernel's "
-                f"butterflies of each kind (harvey {mix['harvey']:.4f}, slack {mix['slack']:.4f}, "
-                f"wide {mix['wide']:.4f})")
+    if rate:
+        mix, ceil = res["butterfly_mix"][name], ceilings[name]
+        out["arith"] = {"achieved": round(rate / 1e9, 2), "peak": round(ceil / 1e9, 2), "unit": "Gbutterfly/s",
+                        "frac": round(rate / ceil, 4),
+                        "butterflies_per_launch": round(bfly[name] * steps / launches),
+                        "peak_source": "measured here, operands in registers (tb_measure_*_butterfly_rate), weighted by "
+                                       "the shares of the kernel's butterflies of each kind: "
+                                       + ", ".join(f"{k} {sh:.4f} at {rates[k] / 1e9:.2f} G/s"
+                                                   for k, sh in mix.items() if sh)}
+        # the machine bound of an exact-quotient integer butterfly: its Shoup product is one
+        # high and two low 64-bit products (the wide form estimates its quotient from 32-bit
+        # products and may pass it; FP64 butterflies run on the FP64 pipe)
+        m = res["mul64"]
+        out["arith"]["integer_machine_bound"] = {
+            "mul_lo_per_s": round(m["lo"] / 1e9, 1), "mul_hi_per_s": round(m["hi"] / 1e9, 1), "unit": "G/s",
+            "butterflies_per_s": round(1.0 / (1.0 / m["hi"] + 2.0 / m["lo"]) / 1e9, 2),
+            "source": "tb_measure_mul64_rate: mul.lo.u64 / mul.hi.u64 in independent chains; "
+                      "bound = 1 / (1/hi + 2/lo) butterflies per second"}
     return out
 
 
@@ -881,14 +859,13 @@ def butterflies_per_step(L):
     return {k: B * v * per for k, v in limbs.items()}
 
 
-def int_ceiling(lib, q, kind="harvey"):
-    """Butterflies per second of the library's lazy butterfly with everything in
-    registers (tb_measure_butterfly_rate): the integer ceiling of the transforms.
-    kind "slack": the butterfly without the conditional subtraction
-    (tb_measure_slack_butterfly_rate); "wide": the no-subtraction form's butterfly with
-    the estimated quotient (tb_measure_wide_butterfly_rate)."""
+def butterfly_rate(lib, q, kind="harvey"):
+    """Butterflies per second of one of the library's butterflies with everything in
+    registers: "harvey" the lazy integer one (tb_measure_butterfly_rate), "slack" the one
+    without the conditional subtraction, "wide" the no-subtraction form's with the
+    estimated quotient, "fp64" the exact FP64 one (moduli below 2^50)."""
     fn = {"harvey": lib.tb_measure_butterfly_rate, "slack": lib.tb_measure_slack_butterfly_rate,
-          "wide": lib.tb_measure_wide_butterfly_rate}[kind]
+          "wide": lib.tb_measure_wide_butterfly_rate, "fp64": lib.tb_measure_fp64_butterfly_rate}[kind]
     fn.argtypes = [ctypes.c_uint64, ctypes.c_void_p, ctypes.POINTER(ctypes.c_double)]
     r = ctypes.c_double(0)
     import tb_capi
@@ -924,35 +901,39 @@ def mul64_rates(lib):
 
 
 def butterfly_mix(moduli, L, logn):
-    """Per forward-transform kernel at the benchmark shape, the shares of its butterflies
-    of each kind: "wide" (no subtraction, estimated quotient: limbs of moduli below 2^57,
-    in the mod-up at most 15 digits), "slack" (the non-subtracting stages of the
-    deferred-reduction form, moduli below 2^60) and "harvey" (its subtracting stages,
-    and every stage above 2^60). Limbs of moduli below 2^50 run in exact FP64 instead (a
-    butterfly rate of 2,274 G/s in registers); the mix states what the integer form of the
-    same transform would run, so their fractions of the integer ceiling may pass 1. The mod-up covers digit j on every key modulus but its
-    own at L data limbs and at L-1 after the rescale; the mod-down and the rescale
-    transform data limbs."""
+    """Per transform kernel at the benchmark shape, the shares of its butterflies of each
+    kind: "fp64" (limbs of moduli below 2^50, N = 4096 .. 32768), and in integer form "wide"
+    (no subtraction, estimated quotient: moduli below 2^57, in the mod-up at most 15
+    digits), "slack" (the non-subtracting stages of the deferred-reduction form, moduli
+    below 2^60) and "harvey" (its subtracting stages, every stage above 2^60, and the
+    inverse transforms). The mod-up covers digit j on every key modulus but its own at L
+    data limbs and at L-1 after the rescale; the mod-down, the rescale and the target
+    inverse transform data limbs, the special and last-limb inverses one limb each."""
     special = moduli[-1]
     sub = fwd_subtracting_stages(logn) / logn
 
-    def kinds(q, wide):
-        if wide and q < (1 << 57):
-            return {"wide": 1.0, "slack": 0.0, "harvey": 0.0}
-        if q < (1 << 60):
-            return {"wide": 0.0, "slack": 1.0 - sub, "harvey": sub}
-        return {"wide": 0.0, "slack": 0.0, "harvey": 1.0}
+    def kinds(q, wide=True, forward=True):
+        if q < (1 << 50) and 12 <= logn <= 15:
+            return {"fp64": 1.0}
+        if forward and wide and q < (1 << 57):
+            return {"wide": 1.0}
+        if forward and q < (1 << 60):
+            return {"slack": 1.0 - sub, "harvey": sub}
+        return {"harvey": 1.0}
 
     def mean(rows):
-        return {k: sum(r[k] for r in rows) / len(rows) for k in ("wide", "slack", "harvey")}
+        return {k: sum(r.get(k, 0.0) for r in rows) / len(rows) for k in ("fp64", "wide", "slack", "harvey")}
 
     up = []
     for lv in (L, L - 1):
         targets = list(moduli[:lv]) + [special]
         up += [kinds(q, lv <= 15) for j in range(lv) for i, q in enumerate(targets) if i != j]
-    down = [kinds(q, True) for lv in (L, L - 1) for q in moduli[:lv]]
-    resc = [kinds(q, True) for q in moduli[:L - 1]]
-    return {"ks_modup_ntt": mean(up), "ks_moddown": mean(down), "rescale_ntt": mean(resc)}
+    data = [q for lv in (L, L - 1) for q in moduli[:lv]]
+    return {"ks_modup_ntt": mean(up), "ks_moddown": mean([kinds(q) for q in data]),
+            "rescale_ntt": mean([kinds(q) for q in moduli[:L - 1]]),
+            "ks_target_intt": mean([kinds(q, forward=False) for q in data]),
+            "ks_special_intt": mean([kinds(special, forward=False)]),
+            "rescale_last_intt": mean([kinds(moduli[L - 1], forward=False)])}
 
 
 TRAFFIC_PROFILE = os.path.join(ROOT, "profiles", "ckks_step_n16384_traffic.md")

@@ -287,7 +287,9 @@ int tb_decrypt(tb_context *ctx, const uint64_t *sk, int L, int size, const uint6
    mod t per plaintext -> n coefficients. Needs an NTT-friendly plain modulus. */
 int tb_batch_encode(tb_context *ctx, const uint64_t *slots, uint64_t slot_stride, uint64_t count, uint64_t *plain,
                     uint64_t batch, void *stream);
-/* BatchEncoderCuda::decode (src/batchencoder_cuda.cu:182-265): n coefficients -> n slots. */
+/* BatchEncoderCuda::decode (src/batchencoder_cuda.cu:182-265): n coefficients -> n slots.
+   slots may overlap plain (overlapped plaintexts are copied first, unless each is replaced
+   by its own slots). */
 int tb_batch_decode(tb_context *ctx, const uint64_t *plain, uint64_t *slots, uint64_t slot_stride, uint64_t batch,
                     void *stream);
 
@@ -430,6 +432,10 @@ int tb_measure_slack_butterfly_rate(uint64_t modulus, void *stream, double *butt
    Shoup quotient is estimated from three 32-bit partial products. No counterpart in the
    reference. */
 int tb_measure_wide_butterfly_rate(uint64_t modulus, void *stream, double *butterflies_per_second);
+/* The same rate for the exact FP64 butterfly of the transforms modulo primes below 2^50
+   (N = 4096 .. 32768); `modulus` odd, 3 <= modulus < 2^50. No counterpart in the
+   reference. */
+int tb_measure_fp64_butterfly_rate(uint64_t modulus, void *stream, double *butterflies_per_second);
 /* The device's 64-bit integer multiply throughput in products per second: kind 0 the
    low word (mul.lo.u64), kind 1 the high word (mul.hi.u64), each in long independent
    chains at full occupancy. A Shoup product is one high and two low products, so

@@ -11,8 +11,9 @@
 //
 // Why: the 64-bit integer Shoup product needs about 14 - 18 issue slots of the FMA-heavy
 // pipe, the FP64 pipe (64 lanes a clock and SM on B200) is idle meanwhile. A whole
-// butterfly is 8 FP64 instructions; measured with operands in registers on B200: 2,274 G
-// butterflies/s against 1,023 G for the estimated-quotient integer butterfly.
+// butterfly is 8 FP64 instructions; measured with operands in registers on B200
+// (tb_measure_fp64_butterfly_rate): 2,200 G butterflies/s against 1,023 G for the
+// estimated-quotient integer butterfly.
 #pragma once
 
 #include <cstdint>
@@ -66,8 +67,8 @@ __device__ __forceinline__ double fp_centred(uint64_t w, uint64_t q) {
     return w > (q >> 1) ? -fp_from_u64(q - w) : fp_from_u64(w);
 }
 
-// Where the pass-ordered tables (FP64, and the integer ones at roots + 2 N) keep the
-// twiddles of the integer tables in natural order. The three stages of a
+// Where the pass-ordered tables (FP64, and the integer ones at roots + 2 N for N <= 2^14)
+// keep the twiddles of the integer tables in natural order. The three stages of a
 // radix-8 pass starting at stage s use 7 consecutive ranges of 2^s twiddles (forward:
 // indices 2^s .. 8 2^s - 1); the ordered tables hold, inside the same range, twiddle k (0 ..
 // 6, in stage order) of every group side by side, so a warp's loads of one k are

@@ -259,7 +259,7 @@ __global__ void ternary_fixup_kernel(const uint8_t *__restrict__ buf, uint64_t b
         uint32_t x;
         do {
             if (p >= avail_words) {
-                s.flag = 2;  // stream window exhausted: reported by prng_check
+                s.flag = 2;  // more rejections (2^-32 a word) than the window has words to spare
                 return;
             }
             x = w[p++];

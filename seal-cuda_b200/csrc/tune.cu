@@ -8,6 +8,8 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdlib>
+#include <cstring>
+#include <string>
 #include <vector>
 
 #include "../../include/troy_b200.h"
@@ -130,7 +132,9 @@ int autotune_ntt(Context &c, uint64_t polys, cudaStream_t s, int *chosen_fwd, in
 // ct_butterfly_slack (the deferred-reduction stages of moduli below 2^60) and KIND 2
 // ct_butterfly_wide (the no-subtraction form with estimated quotients, moduli below
 // 2^57) instead; their values wrap modulo 2^64 over the rounds, which changes no
-// instruction and so not the rate.
+// instruction and so not the rate. KIND 3 times the exact FP64 butterfly (fp64mod.cuh,
+// moduli below 2^50); its values leave the exact range over the rounds, for the largest
+// moduli the finite one too, which changes no instruction either.
 struct Twiddles7 {
     ulonglong2 w[7];
 };
@@ -165,20 +169,58 @@ __global__ void __launch_bounds__(256) butterfly_rate_kernel(uint64_t *sink, Twi
     sink[tid] = x;
 }
 
+// The twiddles' words are the doubles' bits: centred twiddle and quotient.
+template <>
+__global__ void __launch_bounds__(256) butterfly_rate_kernel<3>(uint64_t *sink, Twiddles7 tw, uint64_t q, int rounds) {
+    const double qd = (double)q;
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
+    double v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = (double)((tid * 8u + (uint32_t)k) % q);
+    auto butterfly = [&](double &x, double &y, const ulonglong2 &w) {
+        const double r = fp_mulmod(y, __longlong_as_double((long long)w.x), __longlong_as_double((long long)w.y), qd);
+        y = __dadd_rn(x, -r);
+        x = __dadd_rn(x, r);
+    };
+    for (int r = 0; r < rounds; r++) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) butterfly(v[k], v[k + 4], tw.w[0]);
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (!(k & 2)) butterfly(v[k], v[k + 2], tw.w[1 + (k >> 2)]);
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) butterfly(v[k], v[k + 1], tw.w[3 + (k >> 1)]);
+    }
+    double x = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) x += v[k];
+    sink[tid] = (uint64_t)__double_as_longlong(x);
+}
+
 int measure_butterfly_rate(uint64_t q, int kind, cudaStream_t s, double *rate) {
-    if (!rate || q < 3 || !(q & 1) || q >= (1ull << 61))
-        return set_error(TB_ERR_INVALID_ARGUMENT, "modulus must be odd, at least 3 and below 2^61");
+    const int bits = kind == 3 ? 50 : 61;
+    if (!rate || q < 3 || !(q & 1) || q >> bits)
+        return set_error(TB_ERR_INVALID_ARGUMENT,
+                         "modulus must be odd, at least 3 and below 2^" + std::to_string(bits));
     Twiddles7 tw;
     uint64_t z = 0x9e3779b97f4a7c15ull ^ q;
     for (int i = 0; i < 7; i++) {
         z = z * 6364136223846793005ull + 1442695040888963407ull;
         const uint64_t w = (z >> 3) % q;
         tw.w[i] = make_ulonglong2(w, (uint64_t)(((unsigned __int128)w << 64) / q));
+        if (kind == 3) {
+            const double c = w > q / 2 ? -(double)(q - w) : (double)w, cq = c * (1.0 / (double)q);
+            std::memcpy(&tw.w[i].x, &c, 8);
+            std::memcpy(&tw.w[i].y, &cq, 8);
+        }
     }
     int dev = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const auto kernel = kind == 2 ? butterfly_rate_kernel<2> : kind == 1 ? butterfly_rate_kernel<1> : butterfly_rate_kernel<0>;
+    const auto kernel = kind == 3   ? butterfly_rate_kernel<3>
+                        : kind == 2 ? butterfly_rate_kernel<2>
+                        : kind == 1 ? butterfly_rate_kernel<1>
+                                    : butterfly_rate_kernel<0>;
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, 0);
     if (e != cudaSuccess) return status_from(e);
     const unsigned blocks = (unsigned)(sms * std::max(per_sm, 1));
@@ -276,6 +318,10 @@ int tb_measure_slack_butterfly_rate(uint64_t modulus, void *stream, double *butt
 
 int tb_measure_wide_butterfly_rate(uint64_t modulus, void *stream, double *butterflies_per_second) {
     return tb::measure_butterfly_rate(modulus, 2, (cudaStream_t)stream, butterflies_per_second);
+}
+
+int tb_measure_fp64_butterfly_rate(uint64_t modulus, void *stream, double *butterflies_per_second) {
+    return tb::measure_butterfly_rate(modulus, 3, (cudaStream_t)stream, butterflies_per_second);
 }
 
 int tb_ntt_set_variant(int forward, int log_block, int variant) {

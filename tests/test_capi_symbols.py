@@ -47,6 +47,12 @@ def test_butterfly_rate_refuses_bad_moduli_on_the_host():
         for q in (0, 2, 1 << 40, (1 << 61) + 1):
             assert fn(q, None, ctypes.byref(r)) == 1
         assert b"2^61" in lib.tb_last_error()
+    fp64 = lib.tb_measure_fp64_butterfly_rate
+    fp64.argtypes = [ctypes.c_uint64, ctypes.c_void_p, ctypes.POINTER(ctypes.c_double)]
+    for q in (0, 2, 1 << 40, (1 << 50) + 1):
+        r = ctypes.c_double(0)
+        assert fp64(q, None, ctypes.byref(r)) == 1
+        assert b"2^50" in lib.tb_last_error()
     lib.tb_measure_mul64_rate.argtypes = [ctypes.c_int, ctypes.c_void_p, ctypes.POINTER(ctypes.c_double)]
     r = ctypes.c_double(0)
     for kind in (-1, 2):

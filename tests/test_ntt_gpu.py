@@ -241,6 +241,12 @@ def test_integer_ceiling_is_measured():
         assert 1e10 < r.value < 1e14
         rates.append(r.value)
     assert rates[1] > 0.95 * rates[0] and rates[2] > 0.95 * rates[1]
+    fp64 = lib.tb_measure_fp64_butterfly_rate
+    fp64.argtypes = [ctypes.c_uint64, ctypes.c_void_p, ctypes.POINTER(ctypes.c_double)]
+    for q in ((1 << 40) - 87, (1 << 50) - 27):
+        r = ctypes.c_double(0)
+        tb_capi.check(fp64(q, None, ctypes.byref(r)))
+        assert 1e10 < r.value < 1e14
     # the machine's 64-bit multiply throughputs bound the exact-quotient butterflies: one
     # high and two low 64-bit products each (the wide form estimates its quotient from
     # 32-bit products and is not bound by this)

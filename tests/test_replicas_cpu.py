@@ -1,7 +1,7 @@
 """The host-side parts of bench.py on CPU. Its multi-GPU path (replicas, one process per
 GPU): two gloo ranks with different timings combine to the slowest rank's times and the
 whole-job rate counts both ranks' work; with one rank nothing is exchanged. The reference
-arm without its library."""
+arm without its library, and the butterflies that the ceilings of the transforms count."""
 import os
 import socket
 import sys
@@ -88,3 +88,17 @@ def test_reference_arm_without_its_library(monkeypatch, capsys, tmp_path):
     bench.main()
     line = json.loads(capsys.readouterr().out)
     assert line["impl"] == "reference" and "libtroyref.so" in line["unavailable"]
+
+
+@pytest.mark.parametrize("bits,fp64", [([60] + [40] * 7 + [60], True), ([60] + [55] * 7 + [60], False)])
+def test_transform_ceilings_count_the_butterflies_that_run(bits, fp64):
+    sys.path.insert(0, ROOT)
+    import bench
+    moduli = [(1 << b) - 1 - 2 * i for i, b in enumerate(bits)]   # the sizes matter only
+    mix = bench.butterfly_mix(moduli, 8, 14)
+    assert set(mix) == set(bench.butterflies_per_step(8))
+    assert all(sum(m.values()) == pytest.approx(1.0) for m in mix.values())
+    # the mod-up covers 64 + 49 limbs, of which 49 + 36 modulo one of the seven middle primes
+    assert mix["ks_modup_ntt"]["fp64" if fp64 else "wide"] == pytest.approx(85 / 113)
+    assert mix["ks_special_intt"] == {"fp64": 0, "wide": 0, "slack": 0, "harvey": 1}
+    assert mix["rescale_last_intt"]["fp64"] == (1 if fp64 else 0)
